@@ -31,8 +31,8 @@
 #include <unordered_map>
 #include <vector>
 
-#include "gb_zstd.h"
 #include "gb_agg_host.h"
+#include "gb_inflate.cuh"
 #include "gb_kernels.cuh"
 
 namespace gb {
@@ -1882,8 +1882,9 @@ struct PqScratch {
     size_t img_cap = 0, ijobs_cap = 0, ilvl_cap = 0;
     void *views = nullptr;  // per chunk of the batch: its view (k_pq_views)
     size_t views_cap = 0;
-    void *zjobs = nullptr, *zscratch = nullptr;  // ZSTD pieces and their decoders' tables
-    size_t zjobs_cap = 0, zscratch_cap = 0;
+    // ZSTD pieces, what their steps hand on, and the serial decoders' tables
+    void *zjobs = nullptr, *zwork = nullptr, *zscratch = nullptr;
+    size_t zjobs_cap = 0, zwork_cap = 0, zscratch_cap = 0;
 };
 
 static gb_status grow(void *&p, size_t &cap, size_t need) {
@@ -1924,7 +1925,7 @@ void gb_pq_release_scratch(gb_agg *h) {
     }
     for (void *p : {s->file_dev, s->pages, s->runs, s->page_runs, s->dict_pages, s->col_pages, s->chunks, s->ctl,
                     s->dicts, s->dsrc, s->doffs, s->dbytes, s->dmatch, s->dcounts, s->img, s->ijobs, s->ilvl, s->views, s->zjobs,
-                    s->zscratch})
+                    s->zwork, s->zscratch})
         if (p) cudaFree(p);
     for (void *p : s->out)
         if (p) cudaFree(p);
@@ -2068,222 +2069,91 @@ static gb_status pq_varchar_dict(gb_agg *h, const PqView &V, PqScratch *S, const
 }
 
 // ------------------------------------------------ compressed column chunks
-// One piece of a batch's decompressed image: `src_len` bytes at file offset
-// `src` copied (mode 0), inflated from a raw Snappy block (mode 1, the codec
-// of parquet.cpp:44-90, the vendored snappy 1.2.1) or from ZSTD frames (mode
-// 2, parquet.cpp:693-736) into `dst_len` bytes at image offset `dst`.  lvl_slot != ~0: the piece is a page v1 of an
-// OPTIONAL column, whose first 4 bytes (the level length) go to lvl[slot].
-struct InflateJob {
-    uint64_t src, dst;
-    uint32_t src_len, dst_len;
-    uint32_t mode, lvl_slot;
-};
+// Stored chunks are copied in pieces of this size, each by a block.
+#define PQ_COPY (1u << 18)
+// ZSTD pages are decoded in groups of at most this many page bytes: the
+// scratch of a group is five times its size (literals, and 12 bytes for each
+// three output bytes of sequences).
+#define PZ_GROUP (384ull << 20)
 
-// One warp per piece.  Snappy (the published format): a varint with the
-// uncompressed length, then elements whose tag's low 2 bits say literal (00:
-// length in the tag or in 1-4 following bytes), or copy with a 1-, 2- or
-// 4-byte offset (01/10/11) of an earlier output position, possibly
-// overlapping the bytes it writes.
-//
-// The warp decodes a round of elements at a time.  Lane L reads the 8
-// compressed bytes at ip + L (one aligned word per lane, redistributed by
-// shuffles) and decodes the element a tag there would be; the chain of real
-// tags from ip (each start plus its element's compressed size) is walked with
-// shuffles over the lanes' sizes, up to the first start at or past ip + 32.
-// An exclusive scan of the starts' lengths places each element in the output.
-// Each output byte of the round gets its source in a per-warp shared map: a
-// compressed position (literal) or an earlier output position (copy; an
-// overlapping copy repeats its first `offset` bytes).  A source inside the
-// round is followed through the map to a byte written before the round or a
-// literal byte, so that all bytes of a round are independent and the warp
-// writes them with one load and one store each.  A literal longer than 64
-// bytes (the last element of its round) is copied by the whole warp after
-// the round.  Every length and offset is checked against the piece's bounds;
-// a malformed block sets ERR_CORRUPT and stops.
-#define PQ_INF_MAP 1024   // output bytes of one round: at most 16 elements of at most 64 bytes
-#define PQ_INF_LONG 64    // literals longer than this are copied by the warp
-#define PQ_INF_LIT 0x80000000u
-
-__device__ __forceinline__ void pq_inflate_piece(const uint8_t *__restrict__ file, const InflateJob J, uint8_t *img,
-                                                 uint32_t *lvl, Ctl *ctl, uint32_t *map, const int lane) {
-    const uint8_t *src = file + J.src;
-    uint8_t *dst = img + J.dst;
-    bool bad = false;
-    if (J.mode == 0) {
-        for (uint32_t i = lane; i < J.src_len; i += 32) dst[i] = src[i];
-    } else {
-        const uint32_t slen = J.src_len, dlen = J.dst_len;
-        uint32_t ip = 0, op = 0;
-        if (lane == 0) {  // the preamble: the uncompressed length
-            uint64_t ulen = 0;
-            int sh = 0;
-            for (;;) {
-                if (ip >= slen || sh > 28) {
-                    bad = true;
-                    break;
-                }
-                const uint8_t b = src[ip++];
-                ulen |= (uint64_t)(b & 0x7f) << sh;
-                if (!(b & 0x80)) break;
-                sh += 7;
-            }
-            if (ulen != dlen) bad = true;
+// Decode the ZSTD pieces of a batch into its image.
+static gb_status pq_unzstd(gb_agg *h, PqScratch *S, const uint8_t *dfile, std::vector<InflateJob> &jobs, Ctl *dctl,
+                           cudaStream_t st) {
+    std::stable_sort(jobs.begin(), jobs.end(), [](const InflateJob &a, const InflateJob &b) { return a.dst_len > b.dst_len; });
+    struct Group {
+        size_t first, n;
+        uint64_t bytes, blocks;
+    };
+    std::vector<Group> groups;
+    uint64_t most = 0, most_blocks = 0;
+    size_t most_n = 0;
+    for (size_t k = 0; k < jobs.size();) {
+        Group g{k, 0, 0, 0};
+        for (; k < jobs.size() && (g.n == 0 || g.bytes + jobs[k].dst_len <= PZ_GROUP); k++, g.n++) {
+            jobs[k].aux = g.bytes;
+            jobs[k].blk = (uint32_t)g.blocks;
+            jobs[k].blk_cap = jobs[k].dst_len / 8192 + 4;
+            g.bytes += ((uint64_t)jobs[k].dst_len + 15) & ~15ull;
+            g.blocks += jobs[k].blk_cap;
         }
-        bad = __shfl_sync(FULL, (int)bad, 0) != 0;
-        ip = __shfl_sync(FULL, ip, 0);
-        while (!bad && op < dlen) {
-            if (ip >= slen) {
-                bad = true;
-                break;
-            }
-            // bytes [ip + lane, ip + lane + 8): lanes 0..10 load the aligned words over
-            // [ip, ip + 40) and the warp redistributes them
-            const uint8_t *blk = (const uint8_t *)((uintptr_t)(src + ip) & ~(uintptr_t)3);
-            uint32_t word = 0;
-            if (lane < 11) {
-                const uint8_t *wp = blk + 4 * lane;
-                if (blk >= src && blk + 44 <= src + slen) {
-                    word = __ldg((const uint32_t *)wp);
-                } else {
-                    for (int k = 0; k < 4; k++)
-                        if (wp + k >= src && wp + k < src + slen) word |= (uint32_t)__ldg(wp + k) << (8 * k);
-                }
-            }
-            const uint32_t sh0 = (uint32_t)((uintptr_t)(src + ip) & 3) + (uint32_t)lane;
-            const uint32_t w0 = __shfl_sync(FULL, word, sh0 >> 2);
-            const uint32_t w1 = __shfl_sync(FULL, word, (sh0 >> 2) + 1);
-            const uint32_t w2 = __shfl_sync(FULL, word, (sh0 >> 2) + 2);
-            const uint32_t lo = __funnelshift_r(w0, w1, 8 * (sh0 & 3)), hi = __funnelshift_r(w1, w2, 8 * (sh0 & 3));
-            // the element a tag at ip + lane would be (selects, no branches)
-            const uint32_t tag = lo & 0xffu, t = tag & 3u, l6 = tag >> 2;
-            const uint32_t rest = (lo >> 8) | (hi << 24);  // bytes 1..4 after the tag
-            const uint32_t nb = l6 >= 60 ? l6 - 59 : 0;     // a literal's length bytes
-            const uint32_t lraw = nb ? rest & (0xffffffffu >> (32 - 8 * nb)) : l6;
-            const uint32_t hdr = t == 0 ? 1 + nb : (t == 1 ? 2 : (t == 2 ? 3 : 5));
-            const uint32_t len = t == 0 ? lraw + 1 : (t == 1 ? 4 + (l6 & 7u) : l6 + 1);  // 0 after a wrap
-            const uint32_t off = t == 1 ? ((tag >> 5) << 8) | (rest & 0xffu) : (t == 2 ? rest & 0xffffu : rest);
-            const uint32_t cs = t != 0 ? hdr : (lraw >= 0x7fff0000u ? 0x7fffffffu : hdr + lraw + 1);
-            // the chain of starts from ip
-            const uint32_t avail = min(32u, slen - ip);
-            uint32_t pos = 0, mask = 0;
-            while (pos < avail) {
-                mask |= 1u << pos;
-                pos += __shfl_sync(FULL, cs, pos);
-            }
-            const bool start = (mask >> lane) & 1u;
-            // lengths clamped in the scan (16 starts of at most 2^26 cannot wrap); the one
-            // element that may be longer, a long literal, is the round's last start
-            uint32_t mylen = start ? min(len, 1u << 26) : 0, incl = mylen;
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, incl, d);
-                if (lane >= d) incl += y;
-            }
-            const uint32_t excl = incl - mylen;  // round-relative output position
-            uint32_t total = __shfl_sync(FULL, incl, 31);
-            const uint32_t p = ip + (uint32_t)lane;  // compressed position of this lane's tag
-            const uint64_t o = (uint64_t)op + excl;
-            const bool live = start && o < dlen;  // elements after the last output byte are ignored
-            const bool mybad = live && ((uint64_t)p + cs > slen || len == 0 || o + len > dlen ||
-                                        (t != 0 && (off == 0 || off > o)));
-            if (__any_sync(FULL, mybad)) {
-                bad = true;
-                break;
-            }
-            // outputs past dlen (trailing elements) and the long literal are not mapped
-            if (total > dlen - op) total = dlen - op;
-            const uint32_t lmask = __ballot_sync(FULL, live && t == 0 && len > PQ_INF_LONG);
-            uint32_t mapped = total, lit_at = 0, lit_len = 0, lit_src = 0;
-            if (lmask) {
-                const int ll = __ffs(lmask) - 1;
-                mapped = __shfl_sync(FULL, excl, ll);
-                lit_len = __shfl_sync(FULL, len, ll);
-                lit_src = __shfl_sync(FULL, p + hdr, ll);
-                lit_at = op + mapped;
-                total = mapped + lit_len;
-            }
-            if (mapped > PQ_INF_MAP) {  // unreachable: 16 starts of at most 64 bytes
-                bad = true;
-                break;
-            }
-            if (start && excl < mapped) {
-                // a literal's byte b comes from q + b; a copy's from o - off + (b mod off)
-                const uint32_t base = t == 0 ? PQ_INF_LIT | (p + hdr) : (uint32_t)o - off;
-                const uint32_t per = t == 0 ? 0xffffffffu : off;
-                for (uint32_t b = 0, r = 0; b < len; b++) {
-                    map[excl + b] = base + r;
-                    r = r + 1 == per ? 0 : r + 1;
-                }
-            }
-            __syncwarp();
-            for (uint32_t k = lane; k < mapped; k += 32) {
-                uint32_t s = map[k];
-                while (!(s & PQ_INF_LIT) && s >= op) s = map[s - op];
-                dst[op + k] = (s & PQ_INF_LIT) ? __ldg(src + (s & ~PQ_INF_LIT)) : dst[s];
-            }
-            if (lit_len) {
-                for (uint32_t b = lane; b < lit_len; b += 32) dst[lit_at + b] = __ldg(src + lit_src + b);
-            }
-            __syncwarp();
-            op += total;
-            ip += pos;
-        }
+        most = std::max(most, g.bytes);
+        most_blocks = std::max(most_blocks, g.blocks);
+        most_n = std::max(most_n, g.n);
+        groups.push_back(g);
     }
-    if (bad && lane == 0) atomicOr(&ctl->err, (u32)ERR_CORRUPT);
-    __syncwarp();
-    if (lane == 0 && J.lvl_slot != ~0u) {
-        uint32_t l4 = ~0u;  // too short to hold a level length: corrupt
-        if (!bad && J.dst_len >= 4)
-            l4 = (uint32_t)dst[0] | ((uint32_t)dst[1] << 8) | ((uint32_t)dst[2] << 16) | ((uint32_t)dst[3] << 24);
-        lvl[J.lvl_slot] = l4;
+    const unsigned serial_blocks = (unsigned)std::min<size_t>((most_n + 3) / 4, (size_t)sm_count());
+    // descriptors | block list | per piece: block count, odd list | literals | sequences
+    auto up = [](uint64_t n) { return (n + 255) & ~255ull; };
+    const uint64_t a_blk = up(sizeof(ZWork)), a_list = a_blk + up(most_blocks * sizeof(ZBlk)), a_nblk = a_list + up(most_blocks * 4),
+                   a_odd = a_nblk + up(most_n * 4), a_lit = a_odd + up(most_n * 4), seqs = most / 3 + 1,
+                   a_seq = a_lit + up(most), all = a_seq + 3 * up(seqs * 4);
+    gb_status s;
+    if ((s = grow(S->zjobs, S->zjobs_cap, jobs.size() * sizeof(InflateJob) + 16)) || (s = grow(S->zwork, S->zwork_cap, all)) ||
+        (s = grow(S->zscratch, S->zscratch_cap, (size_t)serial_blocks * 4 * sizeof(gbz::ZsScratch))))
+        return s;
+    static bool attr = false;
+    if (!attr) {
+        GB_CUDA(cudaFuncSetAttribute(k_pz_bytes, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ZByteShared)));
+        attr = true;
     }
-}
-
-// Each warp claims pieces from a counter (the word after the last job, zero
-// at launch) until none is left; the host lists the pieces longest first, so
-// that the long pages start early and no warp idles beside a long one.
-__global__ void __launch_bounds__(256) k_pq_inflate(const uint8_t *__restrict__ file, InflateJob *jobs,
-                                                    uint32_t n, uint8_t *img, uint32_t *lvl, Ctl *ctl) {
-    __shared__ uint32_t s_map[8][PQ_INF_MAP];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *next = (uint32_t *)(jobs + n);
-    for (;;) {
-        uint32_t j = 0;
-        if (lane == 0) j = atomicAdd(next, 1u);
-        j = __shfl_sync(FULL, j, 0);
-        if (j >= n) return;  // the whole warp
-        pq_inflate_piece(file, jobs[j], img, lvl, ctl, s_map[warp], lane);
+    GB_CUDA(cudaMemcpyAsync(S->zjobs, jobs.data(), jobs.size() * sizeof(InflateJob), cudaMemcpyHostToDevice, st));
+    for (const Group &g : groups) {
+        uint8_t *z = (uint8_t *)S->zwork;
+        ZArgs A;
+        memset(&A, 0, sizeof A);
+        A.file = dfile;
+        A.jobs = (InflateJob *)S->zjobs + g.first;
+        A.n = (u32)g.n;
+        A.img = (uint8_t *)S->img;
+        A.lvl = (u32 *)S->ilvl;
+        A.ctl = dctl;
+        A.work = (ZWork *)z;
+        A.blk = (ZBlk *)(z + a_blk);
+        A.list = (u32 *)(z + a_list);
+        A.n_blk = (u32 *)(z + a_nblk);
+        A.odd = (u32 *)(z + a_odd);
+        A.lits = z + a_lit;
+        A.seq_ll = (u32 *)(z + a_seq);
+        A.seq_ml = (u32 *)(z + a_seq + up(seqs * 4));
+        A.seq_off = (u32 *)(z + a_seq + 2 * up(seqs * 4));
+        GB_CUDA(cudaMemsetAsync(A.work, 0, sizeof(ZWork), st));
+        gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pz_blocks", st);
+        k_pz_blocks<<<(unsigned)((g.n + 127) / 128), 128, 0, st>>>(A);
+        gb_agg_prof_end(h, pm, st);
+        pm = gb_agg_prof_begin(h, "k_pz_entropy", st);
+        const size_t warps = (size_t)std::min<uint64_t>(g.blocks, (uint64_t)sm_count() * 28);
+        k_pz_entropy<<<(unsigned)((warps + ZE_WARPS - 1) / ZE_WARPS), ZE_WARPS * 32, 0, st>>>(A);
+        gb_agg_prof_end(h, pm, st);
+        pm = gb_agg_prof_begin(h, "k_pz_bytes", st);
+        k_pz_bytes<<<(unsigned)std::min<size_t>(g.n, (size_t)sm_count() * 3), XT, sizeof(ZByteShared), st>>>(A);
+        gb_agg_prof_end(h, pm, st);
+        pm = gb_agg_prof_begin(h, "k_pz_serial", st);
+        k_pz_serial<<<serial_blocks, 128, 0, st>>>(A, (gbz::ZsScratch *)S->zscratch);
+        gb_agg_prof_end(h, pm, st);
+        GB_CUDA(cudaGetLastError());
+        gb_agg_count_launch(h, 4);
     }
-}
-
-// ZSTD pieces (mode 2): one warp per piece, claimed from a counter (the word
-// after the last job) longest first, decoded by its first lane with the
-// warp's 13.3 KB of tables in `scratch` (a frame is one serial stream;
-// pieces on the lanes of one warp would serialise on their divergent
-// branches).  The tables stay in global memory.  Launch bounds of 5 blocks
-// an SM hold a thread to 96 registers: 20 warps per SM decode at once, which
-// measured faster than 16 warps at 128 registers and than 24 or 32 warps,
-// whose tighter bounds spill.  A frame that does not
-// decode to exactly dst_len bytes sets ERR_CORRUPT.
-__global__ void __launch_bounds__(128, 5) k_pq_unzstd(const uint8_t *__restrict__ file, InflateJob *jobs, uint32_t n,
-                                                   uint8_t *img, uint32_t *lvl, Ctl *ctl, gbz::ZsScratch *scratch) {
-    if ((threadIdx.x & 31) != 0) return;
-    gbz::ZsScratch &Z = scratch[(blockIdx.x * blockDim.x + threadIdx.x) >> 5];
-    uint32_t *next = (uint32_t *)(jobs + n);
-    for (;;) {
-        const uint32_t j = atomicAdd(next, 1u);
-        if (j >= n) return;
-        const InflateJob J = jobs[j];
-        uint8_t *dst = img + J.dst;
-        const int64_t got = gbz::zstd_decompress(file + J.src, J.src_len, dst, J.dst_len, Z);
-        const bool bad = got != (int64_t)J.dst_len;
-        if (bad) atomicOr(&ctl->err, (u32)ERR_CORRUPT);
-        if (J.lvl_slot != ~0u) {
-            uint32_t l4 = ~0u;  // too short to hold a level length: corrupt
-            if (!bad && J.dst_len >= 4)
-                l4 = (uint32_t)dst[0] | ((uint32_t)dst[1] << 8) | ((uint32_t)dst[2] << 16) | ((uint32_t)dst[3] << 24);
-            lvl[J.lvl_slot] = l4;
-        }
-    }
+    return GB_OK;
 }
 
 // Build a batch's decompressed image: per live row group and mapped file
@@ -2316,7 +2186,10 @@ static gb_status pq_inflate_batch(gb_agg *h, const gb_pq_file *f, PqScratch *S, 
             if (ch.codec == 0) {
                 if (ch.size > 0xffffffffull) return pq_corrupt("column chunk size");
                 const uint64_t at = place(ch.size);
-                jobs.push_back({ch.start - base, at, (uint32_t)ch.size, (uint32_t)ch.size, 0u, ~0u});
+                for (uint64_t o = 0; o < ch.size; o += PQ_COPY) {
+                    const uint32_t m = (uint32_t)std::min<uint64_t>(PQ_COPY, ch.size - o);
+                    jobs.push_back({ch.start - base + o, at + o, m, m, 0u, ~0u, 0, 0, 0});
+                }
                 const int64_t d = (int64_t)at - (int64_t)ch.start;
                 if (ch.dict_off >= 0) ch.dict_off += d;
                 for (uint32_t p = ch.page_begin; p < ch.page_end; p++) {
@@ -2328,26 +2201,26 @@ static gb_status pq_inflate_batch(gb_agg *h, const gb_pq_file *f, PqScratch *S, 
             const uint32_t cm = ch.codec == 6 ? 2u : 1u;  // ZSTD or SNAPPY
             if (ch.dict_off >= 0) {
                 const uint64_t at = place(ch.dict_bytes);
-                jobs.push_back({ch.dict_src - base, at, ch.dict_src_bytes, ch.dict_bytes, cm, ~0u});
+                jobs.push_back({ch.dict_src - base, at, ch.dict_src_bytes, ch.dict_bytes, cm, ~0u, 0, 0, 0});
                 ch.dict_off = (int64_t)at;
             }
             for (uint32_t p = ch.page_begin; p < ch.page_end; p++) {
                 PqPage &pg = ip[p];
                 const uint64_t at = place((uint64_t)pg.lvl_copy + pg.raw_bytes);
                 if (pg.lvl_copy) {
-                    jobs.push_back({pg.src_off - pg.lvl_copy - base, at, pg.lvl_copy, pg.lvl_copy, 0u, ~0u});
+                    jobs.push_back({pg.src_off - pg.lvl_copy - base, at, pg.lvl_copy, pg.lvl_copy, 0u, ~0u, 0, 0, 0});
                     pg.def_off = at;
                     pg.def_bytes = pg.lvl_copy;
                 }
                 jobs.push_back({pg.src_off - base, at + pg.lvl_copy, pg.src_bytes, pg.raw_bytes, pg.stored ? 0u : cm,
-                                pg.lvl_pending ? (uint32_t)pending.size() : ~0u});
+                                pg.lvl_pending ? (uint32_t)pending.size() : ~0u, 0, 0, 0});
                 if (pg.lvl_pending) pending.push_back(p);
                 pg.off = at + pg.lvl_copy;
                 pg.bytes = pg.raw_bytes;
             }
         }
     }
-    // the ZSTD pieces in a list of their own (a kernel of their own)
+    // the ZSTD pieces in a list of their own (kernels of their own)
     std::vector<InflateJob> zjobs;
     for (size_t k = 0; k < jobs.size();) {
         if (jobs[k].mode == 2) {
@@ -2359,38 +2232,29 @@ static gb_status pq_inflate_batch(gb_agg *h, const gb_pq_file *f, PqScratch *S, 
         }
     }
     // longest first (a stored piece costs about a sixteenth of an inflated
-    // one per byte), then a zero word: the kernels' claim counters
+    // one per byte), then a zero word: the kernel's claim counter
     auto longest = [](const InflateJob &a, const InflateJob &b) {
         return (a.mode ? (uint64_t)a.dst_len * 16 : a.dst_len) > (b.mode ? (uint64_t)b.dst_len * 16 : b.dst_len);
     };
     std::stable_sort(jobs.begin(), jobs.end(), longest);
-    std::stable_sort(zjobs.begin(), zjobs.end(), longest);
-    const size_t n_jobs = jobs.size(), n_z = zjobs.size();
-    jobs.push_back({0, 0, 0, 0, 0, 0});
-    zjobs.push_back({0, 0, 0, 0, 0, 0});
-    const size_t z_blocks = std::min<size_t>((n_z + 3) / 4, (size_t)sm_count() * 16);  // 4 warps per block
+    const size_t n_jobs = jobs.size();
+    jobs.push_back({0, 0, 0, 0, 0, 0, 0, 0, 0});
     gb_status s;
     if ((s = grow(S->img, S->img_cap, pos + 64)) || (s = grow(S->ijobs, S->ijobs_cap, jobs.size() * sizeof(InflateJob) + 16)) ||
-        (s = grow(S->ilvl, S->ilvl_cap, pending.size() * 4 + 16)) ||
-        (n_z && ((s = grow(S->zjobs, S->zjobs_cap, zjobs.size() * sizeof(InflateJob) + 16)) ||
-                 (s = grow(S->zscratch, S->zscratch_cap, z_blocks * 4 * sizeof(gbz::ZsScratch))))))
+        (s = grow(S->ilvl, S->ilvl_cap, pending.size() * 4 + 16)))
         return s;
-    if (n_z) {
-        GB_CUDA(cudaMemcpyAsync(S->zjobs, zjobs.data(), zjobs.size() * sizeof(InflateJob), cudaMemcpyHostToDevice, st));
-        gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pq_unzstd", st);
-        k_pq_unzstd<<<(unsigned)z_blocks, 128, 0, st>>>(dfile, (InflateJob *)S->zjobs, (uint32_t)n_z,
-                                                         (uint8_t *)S->img, (uint32_t *)S->ilvl, dctl,
-                                                         (gbz::ZsScratch *)S->zscratch);
-        gb_agg_prof_end(h, pm, st);
-        GB_CUDA(cudaGetLastError());
-        gb_agg_count_launch(h, 1);
-    }
+    if (!zjobs.empty() && (s = pq_unzstd(h, S, dfile, zjobs, dctl, st))) return s;
     if (n_jobs) {
+        static bool attr = false;
+        if (!attr) {
+            GB_CUDA(cudaFuncSetAttribute(k_pq_inflate, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SnapShared)));
+            attr = true;
+        }
         GB_CUDA(cudaMemcpyAsync(S->ijobs, jobs.data(), jobs.size() * sizeof(InflateJob), cudaMemcpyHostToDevice, st));
         gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pq_inflate", st);
-        const unsigned grid = (unsigned)std::min<size_t>((n_jobs + 7) / 8, (size_t)sm_count() * 6);
-        k_pq_inflate<<<grid, 256, 0, st>>>(dfile, (InflateJob *)S->ijobs, (uint32_t)n_jobs, (uint8_t *)S->img,
-                                           (uint32_t *)S->ilvl, dctl);
+        const unsigned grid = (unsigned)std::min<size_t>(n_jobs, (size_t)sm_count() * 3);
+        k_pq_inflate<<<grid, XT, sizeof(SnapShared), st>>>(dfile, (InflateJob *)S->ijobs, (uint32_t)n_jobs,
+                                                          (uint8_t *)S->img, (uint32_t *)S->ilvl, dctl);
         gb_agg_prof_end(h, pm, st);
         GB_CUDA(cudaGetLastError());
         gb_agg_count_launch(h, 1);

@@ -299,7 +299,7 @@ ZS_COLD int64_t zs_seq_table(int mode, int which, const uint8_t *src, int64_t n,
 
 // The Huffman table of a literals section: returns the bytes of its
 // description, or -1.
-ZS_COLD int64_t zs_huf_table(const uint8_t *src, int64_t n, ZsScratch &S, int *maxbits) {
+ZS_COLD int64_t zs_huf_table(const uint8_t *src, int64_t n, uint16_t *huf, uint32_t *wtab, int *maxbits) {
     if (n < 1) return -1;
     uint8_t w[256];
     int nw = 0;
@@ -310,27 +310,27 @@ ZS_COLD int64_t zs_huf_table(const uint8_t *src, int64_t n, ZsScratch &S, int *m
         int16_t norm[64];
         int nsym, al;
         const int64_t nc = zs_read_ncount(src + 1, h, 6, 16, norm, &nsym, &al);
-        if (nc < 0 || !zs_fse_build(S.wt, al, norm, nsym)) return -1;
+        if (nc < 0 || !zs_fse_build(wtab, al, norm, nsym)) return -1;
         ZsBack b;
         if (!zs_back_init(b, src + 1 + nc, (int64_t)h - nc)) return -1;
         uint32_t s1 = zs_read(b, al), s2 = zs_read(b, al);
         for (;;) {
             if (nw >= 255) return -1;
-            uint32_t c = S.wt[s1];
+            uint32_t c = wtab[s1];
             w[nw++] = (uint8_t)(c & 0xff);
             s1 = (c >> 16) + zs_read(b, (int)((c >> 8) & 0xff));
             if (b.pos < 0) {
                 if (nw >= 255) return -1;
-                w[nw++] = (uint8_t)(S.wt[s2] & 0xff);
+                w[nw++] = (uint8_t)(wtab[s2] & 0xff);
                 break;
             }
             if (nw >= 255) return -1;
-            c = S.wt[s2];
+            c = wtab[s2];
             w[nw++] = (uint8_t)(c & 0xff);
             s2 = (c >> 16) + zs_read(b, (int)((c >> 8) & 0xff));
             if (b.pos < 0) {
                 if (nw >= 255) return -1;
-                w[nw++] = (uint8_t)(S.wt[s1] & 0xff);
+                w[nw++] = (uint8_t)(wtab[s1] & 0xff);
                 break;
             }
         }
@@ -366,18 +366,18 @@ ZS_COLD int64_t zs_huf_table(const uint8_t *src, int64_t n, ZsScratch &S, int *m
         if (!w[i]) continue;
         const uint32_t len = 1u << (w[i] - 1);
         const uint16_t e = (uint16_t)((i << 8) | (mb + 1 - w[i]));
-        for (uint32_t k = 0; k < len; k++) S.huf[start[w[i]] + k] = e;
+        for (uint32_t k = 0; k < len; k++) huf[start[w[i]] + k] = e;
         start[w[i]] += len;
     }
     *maxbits = mb;
     return used;
 }
 
-ZS_COLD bool zs_huf_stream(const uint8_t *src, int64_t n, const ZsScratch &S, int mb, uint8_t *out, int64_t count) {
+ZS_COLD bool zs_huf_stream(const uint8_t *src, int64_t n, const uint16_t *huf, int mb, uint8_t *out, int64_t count) {
     ZsBack b;
     if (!zs_back_init(b, src, n)) return false;
     for (int64_t i = 0; i < count; i++) {
-        const uint16_t e = S.huf[zs_peek(b, mb)];
+        const uint16_t e = huf[zs_peek(b, mb)];
         out[i] = (uint8_t)(e >> 8);
         b.pos -= e & 0xff;
     }
@@ -469,7 +469,7 @@ ZS_HD bool zs_block(const uint8_t *src, int64_t n, uint8_t *dst, int32_t cap, in
         int64_t cn = csize;
         if (ltype == 2) {
             int mb;
-            const int64_t used = zs_huf_table(c, cn, S, &mb);
+            const int64_t used = zs_huf_table(c, cn, S.huf, S.wt, &mb);
             if (used < 0) return false;
             F.huf_bits = mb;
             c += used;
@@ -479,7 +479,7 @@ ZS_HD bool zs_block(const uint8_t *src, int64_t n, uint8_t *dst, int32_t cap, in
         }
         const bool four = sf != 0;
         if (!four) {
-            if (!zs_huf_stream(c, cn, S, F.huf_bits, lbuf, lsize)) return false;
+            if (!zs_huf_stream(c, cn, S.huf, F.huf_bits, lbuf, lsize)) return false;
         } else {
             if (cn < 6) return false;
             const int64_t s1 = c[0] | (c[1] << 8), s2 = c[2] | (c[3] << 8), s3 = c[4] | (c[5] << 8);
@@ -488,10 +488,10 @@ ZS_HD bool zs_block(const uint8_t *src, int64_t n, uint8_t *dst, int32_t cap, in
             const int64_t seg = (lsize + 3) / 4;
             if (3 * seg > lsize) return false;
             const uint8_t *p = c + 6;
-            if (!zs_huf_stream(p, s1, S, F.huf_bits, lbuf, seg) ||
-                !zs_huf_stream(p + s1, s2, S, F.huf_bits, lbuf + seg, seg) ||
-                !zs_huf_stream(p + s1 + s2, s3, S, F.huf_bits, lbuf + 2 * seg, seg) ||
-                !zs_huf_stream(p + s1 + s2 + s3, s4, S, F.huf_bits, lbuf + 3 * seg, lsize - 3 * seg))
+            if (!zs_huf_stream(p, s1, S.huf, F.huf_bits, lbuf, seg) ||
+                !zs_huf_stream(p + s1, s2, S.huf, F.huf_bits, lbuf + seg, seg) ||
+                !zs_huf_stream(p + s1 + s2, s3, S.huf, F.huf_bits, lbuf + 2 * seg, seg) ||
+                !zs_huf_stream(p + s1 + s2 + s3, s4, S.huf, F.huf_bits, lbuf + 3 * seg, lsize - 3 * seg))
                 return false;
         }
         pos += csize;
