@@ -17,13 +17,42 @@
 
 namespace gb {
 
-constexpr int XT = 512;              // threads of a block
-constexpr int XW = 8192;             // output bytes of a window
-constexpr int XPER = XW / XT;        // consecutive map entries one thread fills
-constexpr int X_MAP = XW + XW / 16;  // map words, one pad word per 16 (a thread's 16 entries start in other banks)
-constexpr u32 X_LIT = 0x80000000u;   // source: a literal (index in the low bits), else an output position
+constexpr int XT = 1024;     // threads of a block
+constexpr int X_CTAS = 1;   // blocks of an SM: 64 registers a thread (two of 32 registers spill and took 1.4 times as long)
+constexpr int XW = 16384;    // output bytes of a window
+constexpr u32 X_HIST = 32768;  // latest output bytes kept in shared memory (most copies reach less far back)
+constexpr u32 X_LIT = 0x80000000u;  // source: a literal (index in the low bits), else an output position
+constexpr u32 X_LONG = 64;   // an element over this length is filled by a warp
+constexpr int X_NLONG = XW / X_LONG + 2;  // at most so many of them touch a window
 
-__device__ __forceinline__ u32 x_at(u32 b) { return b + (b >> 4); }
+struct XLong {
+    u32 at, len, base, period;  // output place (of the batch), bytes, first source, its period (copies)
+};
+struct alignas(16) XShared {
+    u32 map[XW + 8];  // of a window's byte at output position p: entry p - (window's position rounded down to 4)
+    uint8_t hist[X_HIST];
+    XLong lng[X_NLONG];
+    u32 n_long[2];  // this window's, the next one's
+};
+
+// One element's sources into the map of window [w, w + n) of a batch that
+// starts at output position op: its bytes [at, at + len) come from base on,
+// repeating after `period` bytes.
+__device__ __forceinline__ void x_fill(XShared &X, u32 op, u32 w, u32 n, int par, u32 at, u32 len, u32 base, u32 period) {
+    const u32 b0 = max(at, w), b1 = min(at + len, w + n);
+    if (b0 >= b1) return;
+    if (b1 - b0 > X_LONG) {
+        X.lng[atomicAdd(&X.n_long[par], 1u)] = {at, len, base, period};
+        return;
+    }
+    u32 r = b0 - at;
+    if (r >= period) r %= period;
+    u32 *m = X.map + (b0 - w + ((op + w) & 3)), *end = m + (b1 - b0);
+    for (; m < end; m++) {
+        *m = base + r;
+        r = r + 1 == period ? 0 : r + 1;
+    }
+}
 
 // dst[0, n) = src[0, n) by the whole block: words stored aligned, each from
 // the two aligned source words it spans (an aligned word that holds a byte
@@ -43,37 +72,101 @@ __device__ __forceinline__ void x_copy(uint8_t *dst, const uint8_t *src, u32 n) 
     if (threadIdx.x < n - tail) dst[tail + threadIdx.x] = src[tail + threadIdx.x];
 }
 
-// The n bytes of a window that starts at output position w0: sources in
-// `map`, literals at lit.  A source is an earlier position than the byte it
-// feeds, so following it ends; entries are replaced by what they lead to,
-// which shortens the chains of the bytes behind (any value another thread
-// reads meanwhile leads to the same byte).
-__device__ __forceinline__ void x_write(volatile u32 *map, u32 n, u32 w0, uint8_t *dst, const uint8_t *lit) {
-    for (u32 b0 = threadIdx.x; b0 < n; b0 += 4 * XT) {
-        u32 s[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const u32 b = b0 + j * XT;
-            s[j] = X_LIT;
-            if (b < n) {
-                u32 x = map[x_at(b)];
-                if (!(x & X_LIT) && x >= w0) {
-                    do {
-                        x = map[x_at(x - w0)];
-                    } while (!(x & X_LIT) && x >= w0);
-                    map[x_at(b)] = x;
-                }
-                s[j] = x;
+// The n bytes of window [w, w + n) of a batch that starts at output position
+// op, once every element is in the map or on the long list: literals at lit
+// (those with an index of lit_near + [0, near_n) in shared memory at near),
+// earlier output in the ring from position `from` on (until the window itself
+// takes its place), else in dst.  A source is an earlier position than the
+// byte it feeds, so following it ends; entries are replaced by what they lead
+// to, which shortens the chains of the bytes behind (any value another thread
+// reads meanwhile leads to the same byte).  A thread makes four bytes at a
+// time.  Ends with a barrier.
+__device__ __forceinline__ void x_write(XShared &X, u32 w, u32 n, int par, u32 op, uint8_t *dst, const uint8_t *lit,
+                                        const uint8_t *near, u32 lit_near, u32 near_n, u32 &from) {
+    __syncthreads();
+    const u32 nl = X.n_long[par], w0 = op + w, wa = w0 & ~3u;
+    if (threadIdx.x == 0) X.n_long[par ^ 1] = 0;
+    if (nl) {
+        const XLong L0 = X.lng[0];
+        if (nl == 1 && (L0.base & X_LIT) && L0.at <= w && L0.at + L0.len >= w + n) {  // one literal covers the window
+            x_copy(dst + w0, lit + (L0.base & ~X_LIT) + (w - L0.at), n);
+            from = w0 + n;  // not in the ring
+            __syncthreads();
+            return;
+        }
+        for (u32 i = threadIdx.x >> 5; i < nl; i += XT / 32) {
+            const XLong L = X.lng[i];
+            const u32 b0 = max(L.at, w), b1 = min(L.at + L.len, w + n);
+            for (u32 b = b0 + (threadIdx.x & 31); b < b1; b += 32) {
+                u32 r = b - L.at;
+                if (r >= L.period) r %= L.period;
+                X.map[w0 + (b - w) - wa] = L.base + r;
             }
         }
-        uint8_t v[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (b0 + j * XT < n) v[j] = (s[j] & X_LIT) ? __ldg(lit + (s[j] & ~X_LIT)) : dst[s[j]];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (b0 + j * XT < n) dst[w0 + b0 + j * XT] = v[j];
+        __syncthreads();
     }
+    const u32 ring = max(from + X_HIST, w0 + n) - X_HIST;
+    const u32 quads = (w0 - wa + n + 3) >> 2;
+    const bool words = ((uintptr_t)dst & 3) == 0;
+    for (u32 q = threadIdx.x; q < quads; q += XT) {
+        volatile u32 *map = X.map;
+        const uint4 s4 = *(const uint4 *)(X.map + 4 * q);
+        u32 s[4] = {s4.x, s4.y, s4.z, s4.w};
+        const u32 p = wa + 4 * q;
+        // bytes outside the window: any source that ends the search
+        if (p < w0 || p + 4 > w0 + n) {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (p + j < w0 || p + j >= w0 + n) s[j] = X_LIT | lit_near;
+        }
+        // literals count as negative: a source in the window is one at or above w0
+        bool chased = false;
+        while (max(max((int)s[0], (int)s[1]), max((int)s[2], (int)s[3])) >= (int)w0) {
+            chased = true;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if ((int)s[j] >= (int)w0) s[j] = map[s[j] - wa];
+        }
+        if (chased) *(uint4 *)(X.map + 4 * q) = make_uint4(s[0], s[1], s[2], s[3]);
+        u32 v[4];
+        bool far = false;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const u32 i = s[j] & ~X_LIT, k = i - lit_near;
+            const bool is_lit = (s[j] & X_LIT) != 0, ok = is_lit ? k < near_n : i >= ring;
+            v[j] = ok ? *(is_lit ? near + k : X.hist + (i & (X_HIST - 1))) : 0;
+            far |= !ok;
+        }
+        if (far) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const u32 i = s[j] & ~X_LIT;
+                if (s[j] & X_LIT) {
+                    if (i - lit_near >= near_n) v[j] = __ldg(lit + i);
+                } else if (i < ring) {
+                    v[j] = dst[i];
+                }
+            }
+        }
+        if (p >= w0 && p + 4 <= w0 + n) {
+            const u32 x = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
+            *(u32 *)(X.hist + (p & (X_HIST - 1))) = x;
+            if (words) {
+                *(u32 *)(dst + p) = x;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) dst[p + j] = (uint8_t)v[j];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (p + j >= w0 && p + j < w0 + n) {
+                    dst[p + j] = (uint8_t)v[j];
+                    X.hist[(p + j) & (X_HIST - 1)] = (uint8_t)v[j];
+                }
+        }
+    }
+    __syncthreads();
 }
 
 // Exclusive scan of one value per thread over the block; *total gets the sum.
@@ -128,29 +221,28 @@ __device__ __forceinline__ void x_level(const InflateJob &J, const uint8_t *dst,
 // earlier output position, possibly overlapping the bytes it writes.
 //
 // Where an element starts is known only from the one before it.  The block
-// takes SN_C compressed bytes at a time, computes for every position where
-// the element that a tag there would be ends, and follows these jumps in
-// three steps that all positions take at once: to the end of the position's
-// 32 bytes, then of its 256 bytes, then (one thread, 16 hops) through the
-// SN_C bytes; on the way back 16 threads enter the 32-byte pieces and 128
-// threads mark the real starts in them.  A scan of the starts' output
-// lengths places them.
-constexpr int SN_C = 4096;  // compressed bytes parsed at a time
-constexpr int SN_PER = SN_C / XT;
+// takes SN_C compressed bytes at a time, in segments of 64 (an element with
+// its length in the tag spans at most 62).  One lane per segment walks the
+// chain that would begin at the segment's first byte; then it walks from
+// where the segment before ends until it meets that chain, as two chains
+// nearly always do within a few elements: from there on they are the same,
+// and the segment's end does not depend on where it was entered.  One thread
+// follows the segments' ends and walks again only where they did not meet or
+// a long literal skips segments.
+constexpr int SN_C = 8192;  // compressed bytes parsed at a time
+constexpr int SN_SEG = SN_C / 64;
+constexpr int SN_PER = SN_C / XT;   // positions of a thread
+constexpr int SN_EL = SN_PER / 2;   // elements that can start there
 
+constexpr int SN_J = SN_C + 2 * SN_SEG;  // entries of a jump table: 2 pad entries per segment
 struct SnapShared {
-    u32 map[X_MAP];
-    union {
-        struct {
-            uint16_t j[SN_C], j32[SN_C], j256[SN_C];
-        } jump;
-        u32 o[SN_C];  // output place of each position's element (of the next one, where none starts)
-    };
-    u32 words[SN_C / 4 + 4];  // the compressed bytes, as aligned words
-    u32 mask[SN_C / 32];
-    uint16_t ent32[SN_C / 32], ent256[SN_C / 256];
+    XShared x;  // its map holds the jump tables until the elements are known
+    u32 words[SN_C / 4 + 4];           // the compressed bytes, as aligned words
+    u64 mask[SN_SEG];                  // the starts
+    u32 exit[SN_SEG];                  // where a segment's chain leaves it
     u32 sums[XT / 32];
-    u32 next, job, ip, bad;
+    u32 skips[SN_SEG / 32];
+    u32 changed, next, job, ip, bad;
 };
 
 struct SnapElem {
@@ -186,6 +278,92 @@ __device__ __forceinline__ SnapElem sn_decode(const uint8_t *c) {
     return e;
 }
 
+// Barrier of the first SN_SEG threads.
+__device__ __forceinline__ void sn_sync() {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(SN_SEG) : "memory");
+}
+
+// The first segment from s on whose chain does not end in the next one.
+__device__ __forceinline__ u32 sn_skip(const u32 *skips, u32 s) {
+    u32 g = skips[s >> 5] & (0xffffffffu << (s & 31));
+    while (!g) {
+        s = (s | 31) + 1;
+        g = skips[s >> 5];
+    }
+    return (s & ~31u) + __ffs(g) - 1;
+}
+
+__device__ __forceinline__ u32 sn_at(u32 e) { return e + 2 * (e >> 6); }
+
+// The starts of the staged piece into S.mask, by the first SN_SEG threads; S.next:
+// where the last element ends (SN_C or above; 0xffff: beyond what a jump
+// holds).  jump: per position, where an element there ends; jump4: four
+// elements on, but no further than out of the segment.
+__device__ __forceinline__ void sn_starts(SnapShared &S, const uint16_t *jump, const uint16_t *jump4) {
+    const u32 t = threadIdx.x, end = (t + 1) * 64;
+    u32 entry = t * 64, exit = entry;
+    while (exit < end) exit = jump4[sn_at(exit)];
+    S.exit[t] = exit;
+    // enter each segment where the one before it ends, again for those whose entry changed
+    for (int round = 0; round < SN_SEG; round++) {
+        sn_sync();
+        const u32 in = t ? S.exit[t - 1] : 0;
+        const bool again = t && in != entry && (in >> 6) == t;
+        if (t == 0) S.changed = 0;
+        sn_sync();
+        if (again) {
+            entry = in;
+            u32 e = in;
+            while (e < end) e = jump4[sn_at(e)];
+            if (e != exit) {
+                S.changed = 1;
+                S.exit[t] = exit = e;
+            }
+        }
+        sn_sync();
+        if (!S.changed) break;
+    }
+    u64 m = 0;
+    for (u32 e = entry; e < end;) {
+        const u32 next = jump4[sn_at(e)];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (e < end) {
+                m |= 1ull << (e & 63);
+                if (k < 3) e = jump[sn_at(e)];
+            }
+        }
+        e = next;
+    }
+    S.mask[t] = m;
+    // every segment was entered where the one before it ends: all is as it should be, unless one is skipped
+    const unsigned g = __ballot_sync(FULL, t + 1 == SN_SEG || (exit >> 6) != t + 1);
+    if ((t & 31) == 0) S.skips[t >> 5] = g;
+    sn_sync();
+    if (t == 0) {
+        u32 q = sn_skip(S.skips, 0);  // segments up to q are right
+        for (;;) {
+            u32 x = S.exit[q];
+            const u32 to = min(x >> 6, (u32)SN_SEG);
+            for (u32 k = q + 1; k < to; k++) S.mask[k] = 0;
+            if (x >= SN_C) {
+                S.next = x;
+                break;
+            }
+            u64 p = 0;
+            while (x < (to + 1) * 64) {
+                p |= 1ull << (x & 63);
+                x = jump[sn_at(x)];
+            }
+            S.mask[to] = p;
+            q = to;
+            if (x == S.exit[to]) q = sn_skip(S.skips, to);  // the segments behind it stand
+            else S.exit[to] = x;
+        }
+    }
+}
+
 __device__ __forceinline__ bool sn_piece(const uint8_t *src, const u32 slen, uint8_t *dst, const u32 dlen,
                                          SnapShared &S) {
     const u32 t = threadIdx.x;
@@ -207,139 +385,108 @@ __device__ __forceinline__ bool sn_piece(const uint8_t *src, const u32 slen, uin
         S.bad = bad || ulen != dlen;
     }
     __syncthreads();
-    u32 ip = S.ip, op = 0;
+    u32 ip = S.ip, op = 0, from = 0;
+    int par = 0;
     if (S.bad) return false;
+    static_assert(sizeof(S.x.map) >= 3 * SN_J * sizeof(uint16_t), "jump tables in the map");
+    uint16_t *jump = (uint16_t *)S.x.map, *jump2 = jump + SN_J, *jump4 = jump2 + SN_J;
+    if (t == 0) S.x.n_long[0] = 0;
     while (op < dlen) {
         if (ip >= slen) return false;
         const u32 a = (u32)((uintptr_t)(src + ip) & 3);
         const u32 *blk = (const u32 *)(src + ip - a);
         // words with a byte of [ip, slen), up to SN_C + 8 bytes from ip
         for (u32 k = t; k < SN_C / 4 + 3; k += XT) S.words[k] = 4 * (u64)k < (u64)(slen - ip) + a ? __ldg(blk + k) : 0u;
-        if (t < SN_C / 32) S.ent32[t] = 0xffff;
-        if (t < SN_C / 256) S.ent256[t] = 0xffff;
-        if (t == 0) S.next = 0;
         __syncthreads();
         const uint8_t *c = (const uint8_t *)S.words + a;
         const u32 avail = min((u32)SN_C, slen - ip);
 #pragma unroll
         for (int k = 0; k < SN_PER; k++) {
+            const u32 i = t + k * XT, tag = c[i], ty = tag & 3u;
+            u32 cs = ty == 0 ? (tag >> 2) + 2 : 2 + ((0x310u >> (4 * (ty - 1))) & 15u);  // copies: 2, 3, 5 bytes
+            if (tag >= 240 && ty == 0) cs = min(sn_decode(c + i).cs, 0x10000u);
+            jump[sn_at(i)] = (uint16_t)min(i + cs, 0xffffu);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < SN_PER; k++) {
             const u32 i = t + k * XT;
-            const u32 tag = c[i], ty = tag & 3u, l6 = tag >> 2;
-            u32 cs = ty == 0 ? l6 + 2 : (ty == 1 ? 2u : (ty == 2 ? 3u : 5u));
-            if (ty == 0 && l6 >= 60) cs = min(sn_decode(c + i).cs, 0x10000u);
-            S.jump.j[i] = (uint16_t)min(i + cs, 0xffffu);
+            u32 e = jump[sn_at(i)];
+            if (e < (i | 63) + 1) e = jump[sn_at(e)];
+            jump2[sn_at(i)] = (uint16_t)e;
         }
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < SN_PER; k++) {
-            const u32 i = t + k * XT, end = (i | 31) + 1;
-            u32 e = S.jump.j[i];
-            while (e < end) e = S.jump.j[e];
-            S.jump.j32[i] = (uint16_t)e;
+            const u32 i = t + k * XT;
+            u32 e = jump2[sn_at(i)];
+            if (e < (i | 63) + 1) e = jump2[sn_at(e)];
+            jump4[sn_at(i)] = (uint16_t)e;
         }
         __syncthreads();
+        if (t < SN_SEG) sn_starts(S, jump, jump4);
+        __syncthreads();
+        // the elements that start at this thread's positions.  Only the last
+        // one of all can be longer than the compressed bytes it lies in:
+        // lengths are clamped for the scan
+        u32 bits = (u32)(S.mask[t / (64 / SN_PER)] >> (t * SN_PER & 63)) & ((1u << SN_PER) - 1);
+        u32 len[SN_EL], val[SN_EL], sum = 0;
+        bool mybad = false;
+        u32 last = 0;  // compressed position after the last element here
 #pragma unroll
-        for (int k = 0; k < SN_PER; k++) {
-            const u32 i = t + k * XT, end = (i | 255) + 1;
-            u32 e = S.jump.j32[i];
-            while (e < end) e = S.jump.j32[e];
-            S.jump.j256[i] = (uint16_t)e;
-        }
-        __syncthreads();
-        if (t == 0)
-            for (u32 e = 0; e < SN_C; e = S.jump.j256[e]) S.ent256[e >> 8] = (uint16_t)e;
-        __syncthreads();
-        if (t < SN_C / 256)
-            for (u32 e = S.ent256[t]; e < (t + 1) * 256; e = S.jump.j32[e]) S.ent32[e >> 5] = (uint16_t)e;
-        __syncthreads();
-        if (t < SN_C / 32) {
-            u32 m = 0;
-            for (u32 e = S.ent32[t]; e < (t + 1) * 32; e = S.jump.j[e]) m |= 1u << (e & 31);
-            S.mask[t] = m;
-        }
-        __syncthreads();
-        // this thread's SN_PER positions: the starts' lengths and their checks.  Only the last start can be longer
-        // than the compressed bytes it lies in: lengths are clamped for the scan.
-        const u32 i0 = t * SN_PER, bits = (S.mask[i0 >> 5] >> (i0 & 31)) & ((1u << SN_PER) - 1);
-        u32 sum = 0, end = 0;
-#pragma unroll
-        for (int k = 0; k < SN_PER; k++) {
-            if (((bits >> k) & 1u) && i0 + k < avail) {
-                const SnapElem e = sn_decode(c + i0 + k);
-                sum += min(e.len, 1u << 30);
-                end = i0 + k + e.cs;
+        for (int k = 0; k < SN_EL; k++) {
+            len[k] = 0;
+            val[k] = 1;
+            const u32 i = t * SN_PER + __ffs(bits) - 1;
+            if (bits && i < avail) {
+                const SnapElem e = sn_decode(c + i);
+                val[k] = e.lit ? X_LIT | (ip + i + e.hdr) : e.off;
+                len[k] = min(e.len, 1u << 30);
+                last = i + e.cs;
+                // a length of 2^30 or more, or an offset that looks like a literal: never valid in a page below 2 GB
+                if (e.len == 0 || e.len >= (1u << 30) || (!e.lit && (e.off == 0 || (e.off & X_LIT)))) len[k] |= 1u << 30;
+                sum += len[k] & ~(1u << 30);
+                bits &= bits - 1;
+            } else {
+                bits = 0;
             }
         }
         u32 total, o = x_scan(sum, S.sums, &total);
-        bool mybad = false;
+        u32 at = o;
 #pragma unroll
-        for (int k = 0; k < SN_PER; k++) {
-            S.o[i0 + k] = o;
-            if (((bits >> k) & 1u) && i0 + k < avail) {
-                const SnapElem e = sn_decode(c + i0 + k);
-                const u64 at = (u64)op + o;
-                // elements after the last output byte are ignored
-                if (at < dlen && ((u64)ip + i0 + k + e.cs > slen || e.len == 0 || at + e.len > dlen ||
-                                  (!e.lit && (e.off == 0 || e.off > at))))
-                    mybad = true;
-                o += min(e.len, 1u << 30);
-            }
+        for (int k = 0; k < SN_EL; k++) {
+            const u32 l = len[k] & ~(1u << 30);
+            const u64 pos = (u64)op + at;
+            // elements after the last output byte are ignored
+            if (len[k] && pos < dlen && ((len[k] >> 30) || pos + l > dlen || (!(val[k] & X_LIT) && val[k] > pos))) mybad = true;
+            at += l;
         }
-        end = __reduce_max_sync(FULL, end);
-        if ((t & 31) == 0) atomicMax(&S.next, end);
+        if (last && (u64)op + at - 1 < dlen && sum && (u64)ip + last > slen) mybad = true;
         if (__syncthreads_or(mybad)) return false;
         total = min(total, dlen - op);
         for (u32 w = 0; w < total; w += XW) {
             const u32 n = min((u32)XW, total - w);
-            const u32 first = w + t * XPER;
-            bool whole = true;  // one literal covers the window
-            u32 from = 0;
-            if (t * XPER < n) {
-                u32 lo = 0, hi = SN_C;
-                while (hi - lo > 1) {
-                    const u32 mid = (lo + hi) >> 1;
-                    if (S.o[mid] <= first) lo = mid;
-                    else hi = mid;
-                }
-                u32 i = lo, e0 = S.o[i], b = first;
-                SnapElem e = sn_decode(c + i);
-                from = i + e.hdr;
-                whole = e.lit && e0 <= w && (u64)e0 + e.len >= w + n;
-                if (whole) {
-                    from += w - e0;
-                } else {
-                    const u32 stop_all = min(first + XPER, w + n);
-                    for (;;) {
-                        const u32 stop = min(stop_all, e0 + min(e.len, 1u << 30));
-                        if (e.lit) {
-                            u32 s = X_LIT | (ip + i + e.hdr + (b - e0));
-                            for (; b < stop; b++) S.map[x_at(b - w)] = s++;
-                        } else {
-                            const u32 m = b - e0, base = op + e0 - e.off;
-                            u32 r = m < e.off ? m : m % e.off;
-                            for (; b < stop; b++) {
-                                S.map[x_at(b - w)] = base + r;
-                                r = r + 1 == e.off ? 0 : r + 1;
-                            }
-                        }
-                        if (b >= stop_all) break;
-                        i += e.cs;
-                        e0 = S.o[i];
-                        e = sn_decode(c + i);
-                    }
-                }
+            at = o;
+#pragma unroll
+            for (int k = 0; k < SN_EL; k++) {
+                if (len[k])
+                    x_fill(S.x, op, w, n, par, at, len[k], (val[k] & X_LIT) ? val[k] : op + at - val[k],
+                           (val[k] & X_LIT) ? 0xffffffffu : val[k]);
+                at += len[k];
             }
-            if (__syncthreads_and(whole)) {
-                if (t == 0) S.ip = from;
-                __syncthreads();
-                x_copy(dst + op + w, src + ip + S.ip, n);
-            } else {
-                x_write(S.map, n, op + w, dst, src);
-            }
-            __syncthreads();
+            x_write(S.x, w, n, par, op, dst, src, c, ip, SN_C, from);
+            par ^= 1;
         }
         op += total;
-        ip += S.next;
+        if (avail < SN_C) {
+            ip = slen;
+        } else if (S.next >= 0xffff) {  // a literal that jumps do not reach over: it is the last element
+            if (last > SN_C) S.ip = last;
+            __syncthreads();
+            ip += S.ip;
+        } else {
+            ip += S.next;
+        }
         __syncthreads();
     }
     return true;
@@ -347,7 +494,7 @@ __device__ __forceinline__ bool sn_piece(const uint8_t *src, const u32 slen, uin
 
 // Stored and SNAPPY pieces: a block claims pieces from a counter (the word
 // after the last job, zero at launch), longest first, until none is left.
-__global__ void __launch_bounds__(XT, 3) k_pq_inflate(const uint8_t *__restrict__ file, InflateJob *jobs, uint32_t n,
+__global__ void __launch_bounds__(XT, X_CTAS) k_pq_inflate(const uint8_t *__restrict__ file, InflateJob *jobs, uint32_t n,
                                                       uint8_t *img, uint32_t *lvl, Ctl *ctl) {
     extern __shared__ __align__(16) unsigned char x_smem[];
     SnapShared &S = *(SnapShared *)x_smem;
@@ -538,21 +685,20 @@ __global__ void __launch_bounds__(128) k_pz_blocks(const __grid_constant__ ZArgs
 
 // One warp's tables.  The Huffman table is used up before the sequence
 // tables are built.
-constexpr int ZE_WARPS = 4;
+
 constexpr int Z_LL = 0, Z_OF = 512, Z_ML = 768, Z_CELLS = 1280;
 struct alignas(16) ZTables {  // the ring is written 16 bytes at a time
     union {
         uint16_t huf[1u << gbz::ZS_HUF_LOG];
-        // sequence cells: next state's baseline (16 bits) | its bits (8) | its bits + the code's extra bits (8)
+        // sequence cells: the next state's bits (5 bits) | the code's extra bits (6) | 0 | the next state's baseline
+        // from bit 21 on.  The sum of three cells holds the sums of the bits in the same places.
         u32 cell[Z_CELLS];
     };
     union {
         u32 wt[64];
         u32 ring[256];  // two 512-byte pieces of the sequences' bit stream
     };
-    uint8_t sym[Z_CELLS];
-    int q[32];      // per sequence of a batch: stream position before it, and its three states
-    u32 state[32];
+    u32 val[Z_CELLS];  // per cell: the code's baseline (24 bits) | its extra bits (8)
     int log[3], at, bad;
 };
 
@@ -645,13 +791,15 @@ __device__ __forceinline__ bool pz_literals(const ZArgs &A, const ZBlk &b, uint8
     return __all_sync(FULL, ok);
 }
 
-// The sequences of block b into the scratch, by one warp: the first lane
-// follows the three states through the bit stream, noting each sequence's
-// position and states, 32 at a time; then every lane reads one sequence's
-// extra bits.  The stream is kept in shared memory, the next 512 bytes
-// already in registers.  What bounds it: the first lane's chain of one table
-// load, the bit count's addition and the extraction of the next states per
-// sequence.
+// The sequences of block b into the scratch, by one warp.  The three states
+// are followed through the bit stream by all lanes alike (the loads are
+// broadcasts and nothing diverges), lane k keeping the position and states of
+// the k-th of 32 sequences; then every lane reads its sequence's extra bits.
+// The stream is kept in shared memory, the next 512 bytes already in
+// registers.  What bounds it: the chain from a sequence's cells over the sum
+// of their bit counts and the extraction of the next states to the next
+// cells; the 64 bits below the position are therefore loaded beside the
+// cells.
 __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, ZTables &T, int lane) {
     if (lane == 0) T.bad = !pz_tables(A, b, T);
     __syncwarp();
@@ -661,12 +809,12 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
         const int at = x == 0 ? Z_LL : (x == 1 ? Z_OF : Z_ML);
         for (int i = lane; i < (1 << T.log[x]); i += 32) {
             const u32 c = T.cell[at + i], s = c & 0xffu, nb = (c >> 8) & 0xffu;
-            u32 xb;
+            u32 xb = 0;
             int xn = (int)s;
             if (x == 0) gbz::zs_ll(s, &xb, &xn);
             if (x == 2) gbz::zs_ml(s, &xb, &xn);
-            T.cell[at + i] = (c >> 16) | (nb << 16) | ((nb + (u32)xn) << 24);
-            T.sym[at + i] = (uint8_t)s;
+            T.cell[at + i] = nb | ((u32)xn << 5) | ((c >> 16) << 21);
+            T.val[at + i] = xb | ((u32)xn << 24);
         }
     }
     const uint8_t *sb = A.file + b.src + T.at;
@@ -690,16 +838,13 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
     ((uint4 *)T.ring)[(low & 1) * 32 + lane] = load(low);
     uint4 ahead = load(low - 1);
     __syncwarp();
-    u32 sl = 0, so = 0, sm = 0;
-    if (lane == 0) {
-        q -= T.log[0];
-        sl = z_rd(T.ring, q, T.log[0]);
-        q -= T.log[1];
-        so = z_rd(T.ring, q, T.log[1]);
-        q -= T.log[2];
-        sm = z_rd(T.ring, q, T.log[2]);
-    }
-    q = __shfl_sync(FULL, q, 0);
+    u32 sl, so, sm;
+    q -= T.log[0];
+    sl = z_rd(T.ring, q, T.log[0]);
+    q -= T.log[1];
+    so = z_rd(T.ring, q, T.log[1]);
+    q -= T.log[2];
+    sm = z_rd(T.ring, q, T.log[2]);
     u32 r0 = b.first ? 1 : Z_SYM, r1 = b.first ? 4 : Z_SYM | (1u << 29), r2 = b.first ? 8 : Z_SYM | (2u << 29);
     u64 lits = 0;
     bool bad = false;
@@ -713,55 +858,48 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
             ahead = load(low - 1);
         }
         __syncwarp();
-        if (lane == 0) {
-            const bool final = k0 + 32 >= nseq;
-            for (int k = 0; k < cnt; k++) {
-                // the 64 bits below q, loaded beside the cells
-                const int w = (q - 64) >> 5;
-                const u32 a0 = T.ring[w & 255], a1 = T.ring[(w + 1) & 255], a2 = T.ring[(w + 2) & 255];
-                const u32 cl = T.cell[Z_LL + sl], co = T.cell[Z_OF + so], cm = T.cell[Z_ML + sm];
-                T.q[k] = q;
-                T.state[k] = sl | (sm << 9) | (so << 18);
-                const u32 nl = (cl >> 16) & 0xffu, nm = (cm >> 16) & 0xffu, no = (co >> 16) & 0xffu;
-                const int take = (int)((cl >> 24) + (co >> 24) + (cm >> 24));
-                if (final && k + 1 == cnt) {  // the last sequence: no next states
-                    q -= take - (int)(nl + nm + no);
-                    break;
-                }
-                q -= take;
-                u32 v = 0;
-                if (take <= 64) {
-                    const u32 sh = (u32)(q + take) & 31;
-                    const u64 win = ((u64)__funnelshift_r(a1, a2, sh) << 32) | __funnelshift_r(a0, a1, sh);
-                    if (take) v = (u32)(win >> (64 - take));
-                } else {
-                    const int ww = q >> 5;
-                    v = __funnelshift_r(T.ring[ww & 255], T.ring[(ww + 1) & 255], q & 31);
-                }
-                so = (co & 0xffffu) + (v & ((1u << no) - 1));
-                sm = (cm & 0xffffu) + ((v >> no) & ((1u << nm) - 1));
-                sl = (cl & 0xffffu) + ((v >> (no + nm)) & ((1u << nl) - 1));
+        int my_q = 0;
+        u32 my_l = 0, my_o = 0, my_m = 0;
+#pragma unroll 2
+        for (int k = 0; k < cnt; k++) {
+            const u32 cl = T.cell[Z_LL + sl], co = T.cell[Z_OF + so], cm = T.cell[Z_ML + sm];
+            // the 96 bits below q (at most 63 + 26 are read)
+            const int w = (q >> 5) - 3;
+            const u32 a0 = T.ring[w & 255], a1 = T.ring[(w + 1) & 255], a2 = T.ring[(w + 2) & 255], a3 = T.ring[(w + 3) & 255];
+            const u32 h0 = __funnelshift_r(a0, a1, (u32)q), h1 = __funnelshift_r(a1, a2, (u32)q), h2 = __funnelshift_r(a2, a3, (u32)q);
+            if (k == lane) {
+                my_q = q;
+                my_l = sl;
+                my_o = so;
+                my_m = sm;
             }
+            const u32 all = cl + co + cm, extra = (all >> 5) & 63;
+            q -= (int)((all & 31) + extra);
+            // the next states' bits, LL, ML, OF from the top: shifts take a cell's low 5 bits
+            const u32 head = __funnelshift_l(extra < 32 ? h1 : h0, extra < 32 ? h2 : h1, extra);
+            sl = (cl >> 21) + __funnelshift_l(head, 0u, cl);
+            const u32 h_m = __funnelshift_l(0u, head, cl);
+            sm = (cm >> 21) + __funnelshift_l(h_m, 0u, cm);
+            so = (co >> 21) + __funnelshift_l(__funnelshift_l(0u, h_m, cm), 0u, co);
         }
-        __syncwarp();
+        // after the last sequence no next states are read: their bits are not there
+        if (k0 + 32 >= nseq) {
+            const u32 n = (T.cell[Z_LL + my_l] + T.cell[Z_OF + my_o] + T.cell[Z_ML + my_m]) & 31;
+            q += (int)__shfl_sync(FULL, n, cnt - 1);
+        }
         u32 ll = 0, ml = 0, off = 4;  // off: the offset value until resolved
         if (lane < cnt) {
-            const u32 st = T.state[lane];
-            u32 lb, mb;
-            int xl, xm;
-            const int xo = T.sym[Z_OF + (st >> 18)];
-            gbz::zs_ll(T.sym[Z_LL + (st & 511)], &lb, &xl);
-            gbz::zs_ml(T.sym[Z_ML + ((st >> 9) & 511)], &mb, &xm);
-            int p = T.q[lane] - xo;
+            const u32 vl = T.val[Z_LL + my_l], vm = T.val[Z_ML + my_m];
+            const int xo = (int)(T.val[Z_OF + my_o] >> 24), xm = (int)(vm >> 24), xl = (int)(vl >> 24);
+            int p = my_q - xo;
             off = (1u << xo) + z_rd(T.ring, p, xo);
             p -= xm;
-            ml = mb + z_rd(T.ring, p, xm);
+            ml = (vm & 0xffffffu) + z_rd(T.ring, p, xm);
             p -= xl;
-            ll = lb + z_rd(T.ring, p, xl);
+            ll = (vl & 0xffffffu) + z_rd(T.ring, p, xl);
             if (off > 3 && ((off - 3) & Z_SYM)) bad = true;
         }
         lits += __reduce_add_sync(FULL, ll);
-        q = __shfl_sync(FULL, q, 0);
         if (!__any_sync(FULL, off <= 3)) {  // every offset is a new one
             off -= 3;
             const u32 n0 = __shfl_sync(FULL, off, cnt - 1), n1 = __shfl_sync(FULL, off, max(cnt - 2, 0)),
@@ -807,17 +945,16 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
     return !__any_sync(FULL, bad) && q == q_end && lits <= b.lsize;
 }
 
-__global__ void __launch_bounds__(ZE_WARPS * 32) k_pz_entropy(const __grid_constant__ ZArgs A) {
+__global__ void __launch_bounds__(32) k_pz_entropy(const __grid_constant__ ZArgs A) {
     static_assert(sizeof(ZTables) % 16 == 0 && offsetof(ZTables, ring) % 16 == 0, "ring alignment");
-    __shared__ ZTables s_tab[ZE_WARPS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    ZTables &T = s_tab[warp];
+    __shared__ ZTables T;
+    const int lane = threadIdx.x;
     const u32 n = A.work->n_list;
     for (;;) {
         u32 i = 0;
         if (lane == 0) i = atomicAdd(&A.work->claim_entropy, 1u);
         i = __shfl_sync(FULL, i, 0);
-        if (i >= n) return;  // the whole warp
+        if (i >= n) return;
         ZBlk &b = A.blk[A.list[i]];
         const InflateJob &J = A.jobs[b.piece];
         bool ok = true;
@@ -836,8 +973,7 @@ __global__ void __launch_bounds__(ZE_WARPS * 32) k_pz_entropy(const __grid_const
 
 constexpr int ZB_SEQ = 2 * XT;  // sequences of a batch
 struct ZByteShared {
-    u32 map[X_MAP];
-    u32 o[ZB_SEQ + 1], l[ZB_SEQ + 1], off[ZB_SEQ];  // per sequence: output place, literal place, offset
+    XShared x;
     u64 sums[XT / 32];
     u32 job;
 };
@@ -850,89 +986,70 @@ __device__ __forceinline__ u32 z_offset(u32 v, u32 r0, u32 r1, u32 r2) {
 
 // One compressed block's bytes at dst + op.
 __device__ __forceinline__ bool pz_block_bytes(const ZArgs &A, const InflateJob &J, const ZBlk &b, uint8_t *dst, u32 &op,
-                                               u32 r0, u32 r1, u32 r2, ZByteShared &S) {
+                                               u32 &from, int &par, u32 r0, u32 r1, u32 r2, ZByteShared &S) {
     const u32 t = threadIdx.x, cap = J.dst_len;
     if (b.bad) return false;
     const uint8_t *lit = b.lit_kind == 0 ? A.file + b.src + b.lit_hdr : A.lits + J.aux + b.lit_off;
-    const u64 base = J.aux / 3 + b.seq_off;
+    const u64 base = J.aux / 3 + b.seq_off + 2 * t;
+    const u32 nseq = b.nseq, lsize = b.lsize;
     u32 lp = 0;
-    for (u32 k0 = 0; k0 < b.nseq; k0 += ZB_SEQ) {
-        const u32 cnt = min((u32)ZB_SEQ, b.nseq - k0);
-        u32 ll[2] = {0, 0}, ml[2] = {0, 0}, off[2] = {0, 0};
+    u32 ll[2], ml[2], off[2];
+    auto load = [&](u32 k0) {
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-            const u32 i = 2 * t + k;
-            if (i < cnt) {
-                ll[k] = A.seq_ll[base + k0 + i];
-                ml[k] = A.seq_ml[base + k0 + i];
-                off[k] = z_offset(A.seq_off[base + k0 + i], r0, r1, r2);
+            ll[k] = ml[k] = off[k] = 0;
+            if (k0 + 2 * t + k < nseq) {
+                ll[k] = A.seq_ll[base + k0 + k];
+                ml[k] = A.seq_ml[base + k0 + k];
+                off[k] = z_offset(A.seq_off[base + k0 + k], r0, r1, r2);
             }
         }
+    };
+    for (u32 k0 = 0; k0 < nseq; k0 += ZB_SEQ) {
+        load(k0);
         // output places in the low half, literal places in the high half
         u64 total;
-        u64 at = x_scan((u64)(ll[0] + ml[0] + ll[1] + ml[1]) | ((u64)(ll[0] + ll[1]) << 32), S.sums, &total);
+        const u64 at = x_scan((u64)(ll[0] + ml[0] + ll[1] + ml[1]) | ((u64)(ll[0] + ll[1]) << 32), S.sums, &total);
+        u32 o = (u32)at, l = lp + (u32)(at >> 32);
         bool bad = false;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-            const u32 i = 2 * t + k, o = (u32)at, l = (u32)(at >> 32);
-            S.o[i] = o;
-            S.l[i] = l;
-            S.off[i] = off[k];
-            if (i < cnt)
-                bad |= (u64)lp + l + ll[k] > b.lsize || (u64)op + o + ll[k] + ml[k] > cap || off[k] == 0 ||
-                       off[k] > op + o + ll[k];
-            at += (u64)(ll[k] + ml[k]) | ((u64)ll[k] << 32);
-        }
-        if (t == 0) {
-            S.o[ZB_SEQ] = (u32)total;
-            S.l[ZB_SEQ] = (u32)(total >> 32);
+            if (k0 + 2 * t + k < nseq)
+                bad |= (u64)l + ll[k] > lsize || (u64)op + o + ll[k] + ml[k] > cap || off[k] == 0 || off[k] > op + o + ll[k];
+            o += ll[k] + ml[k];
+            l += ll[k];
         }
         if (__syncthreads_or(bad)) return false;
         const u32 all = (u32)total;
         for (u32 w = 0; w < all; w += XW) {
             const u32 n = min((u32)XW, all - w);
-            if (t * XPER < n) {
-                u32 bt = w + t * XPER;
-                const u32 stop_all = min(bt + XPER, w + n);
-                u32 i = 0, hi = ZB_SEQ;
-                while (hi - i > 1) {
-                    const u32 mid = (i + hi) >> 1;
-                    if (S.o[mid] <= bt) i = mid;
-                    else hi = mid;
-                }
-                for (;; i++) {
-                    const u32 e0 = S.o[i], l0 = S.l[i], mat = e0 + (S.l[i + 1] - l0), end = min(S.o[i + 1], stop_all);
-                    if (bt < mat) {
-                        const u32 stop = min(mat, stop_all);
-                        u32 s = X_LIT | (lp + l0 + (bt - e0));
-                        for (; bt < stop; bt++) S.map[x_at(bt - w)] = s++;
-                    }
-                    if (bt < end) {
-                        const u32 of = S.off[i], m = bt - mat, from = op + mat - of;
-                        u32 r = m < of ? m : m % of;
-                        for (; bt < end; bt++) {
-                            S.map[x_at(bt - w)] = from + r;
-                            r = r + 1 == of ? 0 : r + 1;
-                        }
-                    }
-                    if (bt >= stop_all) break;
-                }
+            o = (u32)at;
+            l = lp + (u32)(at >> 32);
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                x_fill(S.x, op, w, n, par, o, ll[k], X_LIT | l, 0xffffffffu);
+                o += ll[k];
+                l += ll[k];
+                x_fill(S.x, op, w, n, par, o, ml[k], op + o - off[k], off[k]);
+                o += ml[k];
             }
-            __syncthreads();
-            x_write(S.map, n, op + w, dst, lit);
-            __syncthreads();
+            x_write(S.x, w, n, par, op, dst, lit, S.x.hist, lsize, 1, from);
+            par ^= 1;
         }
         op += all;
         lp += (u32)(total >> 32);
     }
-    const u32 rest = b.lsize - lp;  // lp <= lsize: checked above
+    const u32 rest = lsize - lp;  // lp <= lsize: checked above
     if (rest > cap - op) return false;
-    x_copy(dst + op, lit + lp, rest);
-    op += rest;
+    if (rest) {
+        x_copy(dst + op, lit + lp, rest);
+        op += rest;
+        from = op;  // not in the ring
+    }
     return true;
 }
 
-__global__ void __launch_bounds__(XT, 3) k_pz_bytes(const __grid_constant__ ZArgs A) {
+__global__ void __launch_bounds__(XT, X_CTAS) k_pz_bytes(const __grid_constant__ ZArgs A) {
     extern __shared__ __align__(16) unsigned char x_smem[];
     ZByteShared &S = *(ZByteShared *)x_smem;
     for (;;) {
@@ -944,11 +1061,14 @@ __global__ void __launch_bounds__(XT, 3) k_pz_bytes(const __grid_constant__ ZArg
         const InflateJob J = A.jobs[j];
         uint8_t *dst = A.img + J.dst;
         bool ok = nb != 0;
-        u32 op = 0, r0 = 1, r1 = 4, r2 = 8;
+        u32 op = 0, from = 0, r0 = 1, r1 = 4, r2 = 8;
+        int par = 0;
+        if (threadIdx.x == 0) S.x.n_long[0] = 0;
+        __syncthreads();
         for (u32 k = 0; ok && k < nb; k++) {
             const ZBlk &b = A.blk[J.blk + k];
             if (b.type == 2) {
-                ok = pz_block_bytes(A, J, b, dst, op, r0, r1, r2, S);
+                ok = pz_block_bytes(A, J, b, dst, op, from, par, r0, r1, r2, S);
                 const u32 n0 = z_offset(b.rep[0], r0, r1, r2), n1 = z_offset(b.rep[1], r0, r1, r2),
                           n2 = z_offset(b.rep[2], r0, r1, r2);
                 r0 = n0;
@@ -964,6 +1084,7 @@ __global__ void __launch_bounds__(XT, 3) k_pz_bytes(const __grid_constant__ ZArg
                     for (u32 i = threadIdx.x; i < b.size; i += XT) dst[op + i] = v;
                 }
                 op += b.size;
+                from = op;
             }
             __syncthreads();
         }

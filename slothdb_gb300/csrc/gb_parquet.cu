@@ -2082,19 +2082,20 @@ static gb_status pq_unzstd(gb_agg *h, PqScratch *S, const uint8_t *dfile, std::v
     std::stable_sort(jobs.begin(), jobs.end(), [](const InflateJob &a, const InflateJob &b) { return a.dst_len > b.dst_len; });
     struct Group {
         size_t first, n;
-        uint64_t bytes, blocks;
+        uint64_t bytes, blocks, full;
     };
     std::vector<Group> groups;
     uint64_t most = 0, most_blocks = 0;
     size_t most_n = 0;
     for (size_t k = 0; k < jobs.size();) {
-        Group g{k, 0, 0, 0};
+        Group g{k, 0, 0, 0, 0};
         for (; k < jobs.size() && (g.n == 0 || g.bytes + jobs[k].dst_len <= PZ_GROUP); k++, g.n++) {
             jobs[k].aux = g.bytes;
             jobs[k].blk = (uint32_t)g.blocks;
             jobs[k].blk_cap = jobs[k].dst_len / 8192 + 4;
             g.bytes += ((uint64_t)jobs[k].dst_len + 15) & ~15ull;
             g.blocks += jobs[k].blk_cap;
+            g.full += jobs[k].dst_len / gbz::ZS_BLOCK_MAX + 1;
         }
         most = std::max(most, g.bytes);
         most_blocks = std::max(most_blocks, g.blocks);
@@ -2141,11 +2142,13 @@ static gb_status pq_unzstd(gb_agg *h, PqScratch *S, const uint8_t *dfile, std::v
         k_pz_blocks<<<(unsigned)((g.n + 127) / 128), 128, 0, st>>>(A);
         gb_agg_prof_end(h, pm, st);
         pm = gb_agg_prof_begin(h, "k_pz_entropy", st);
-        const size_t warps = (size_t)std::min<uint64_t>(g.blocks, (uint64_t)sm_count() * 28);
-        k_pz_entropy<<<(unsigned)((warps + ZE_WARPS - 1) / ZE_WARPS), ZE_WARPS * 32, 0, st>>>(A);
+        // one-warp blocks, as many as an encoder that fills its 128 KB blocks makes (more wait their turn), 20 an SM
+        // at most: evenly spread, a warp's serial chain has its scheduler to itself and at most four others
+        const uint64_t warps = std::min<uint64_t>(g.full, (uint64_t)sm_count() * 20);
+        k_pz_entropy<<<(unsigned)warps, 32, 0, st>>>(A);
         gb_agg_prof_end(h, pm, st);
         pm = gb_agg_prof_begin(h, "k_pz_bytes", st);
-        k_pz_bytes<<<(unsigned)std::min<size_t>(g.n, (size_t)sm_count() * 3), XT, sizeof(ZByteShared), st>>>(A);
+        k_pz_bytes<<<(unsigned)std::min<size_t>(g.n, (size_t)sm_count() * X_CTAS), XT, sizeof(ZByteShared), st>>>(A);
         gb_agg_prof_end(h, pm, st);
         pm = gb_agg_prof_begin(h, "k_pz_serial", st);
         k_pz_serial<<<serial_blocks, 128, 0, st>>>(A, (gbz::ZsScratch *)S->zscratch);
@@ -2252,7 +2255,7 @@ static gb_status pq_inflate_batch(gb_agg *h, const gb_pq_file *f, PqScratch *S, 
         }
         GB_CUDA(cudaMemcpyAsync(S->ijobs, jobs.data(), jobs.size() * sizeof(InflateJob), cudaMemcpyHostToDevice, st));
         gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pq_inflate", st);
-        const unsigned grid = (unsigned)std::min<size_t>(n_jobs, (size_t)sm_count() * 3);
+        const unsigned grid = (unsigned)std::min<size_t>(n_jobs, (size_t)sm_count() * X_CTAS);
         k_pq_inflate<<<grid, XT, sizeof(SnapShared), st>>>(dfile, (InflateJob *)S->ijobs, (uint32_t)n_jobs,
                                                           (uint8_t *)S->img, (uint32_t *)S->ilvl, dctl);
         gb_agg_prof_end(h, pm, st);
