@@ -13,9 +13,9 @@
 //
 // 8M-row file of INT32 dictionary, INT16 and INT64 PLAIN columns (1M-row
 // groups, 65,536-row pages, 113 MB of page bytes): SNAPPY 20.0 -> 1.16 ms,
-// ZSTD 50.8 -> 3.24 ms (blocks 0.02, entropy 2.57, bytes 0.65 ms) against one
+// ZSTD 50.8 -> 3.10 ms (blocks 0.02, entropy 2.43, bytes 0.65 ms) against one
 // warp per page.  What is left is the chain of the longest page: 50 pieces of
-// 8 KB (SNAPPY), a block of 31,600 sequences at ~120 cycles each (ZSTD).
+// 8 KB (SNAPPY), a block of 31,600 sequences at ~115 cycles each (ZSTD).
 #pragma once
 
 #include "gb_kernels.cuh"
@@ -696,8 +696,8 @@ constexpr int Z_LL = 0, Z_OF = 512, Z_ML = 768, Z_CELLS = 1280;
 struct alignas(16) ZTables {  // the ring is written 16 bytes at a time
     union {
         uint16_t huf[1u << gbz::ZS_HUF_LOG];
-        // sequence cells: the next state's bits (5 bits) | the code's extra bits (6) | 0 | the next state's baseline
-        // from bit 21 on.  The sum of three cells holds the sums of the bits in the same places.
+        // sequence cells: the next state's bits (5 bits) | the code's extra bits (6) | 0 | four times the next state's
+        // baseline from bit 19 on.  The sum of three cells holds the sums of the bits in the same places.
         u32 cell[Z_CELLS];
     };
     union {
@@ -819,7 +819,7 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
             int xn = (int)s;
             if (x == 0) gbz::zs_ll(s, &xb, &xn);
             if (x == 2) gbz::zs_ml(s, &xb, &xn);
-            T.cell[at + i] = nb | ((u32)xn << 5) | ((c >> 16) << 21);
+            T.cell[at + i] = nb | ((u32)xn << 5) | ((c >> 16) << 21);  // (base * 4) << 19
             T.val[at + i] = xb | ((u32)xn << 24);
         }
     }
@@ -851,6 +851,9 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
     so = z_rd(T.ring, q, T.log[1]);
     q -= T.log[2];
     sm = z_rd(T.ring, q, T.log[2]);
+    sl *= 4;  // states are kept as byte offsets of their cells
+    so *= 4;
+    sm *= 4;
     u32 r0 = b.first ? 1 : Z_SYM, r1 = b.first ? 4 : Z_SYM | (1u << 29), r2 = b.first ? 8 : Z_SYM | (2u << 29);
     u64 lits = 0;
     bool bad = false;
@@ -866,9 +869,10 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
         __syncwarp();
         int my_q = 0;
         u32 my_l = 0, my_o = 0, my_m = 0;
-#pragma unroll 2
-        for (int k = 0; k < cnt; k++) {
-            const u32 cl = T.cell[Z_LL + sl], co = T.cell[Z_OF + so], cm = T.cell[Z_ML + sm];
+        auto step = [&](int k) {
+            const u32 cl = *(const u32 *)((const char *)(T.cell + Z_LL) + sl);
+            const u32 co = *(const u32 *)((const char *)(T.cell + Z_OF) + so);
+            const u32 cm = *(const u32 *)((const char *)(T.cell + Z_ML) + sm);
             // the 96 bits below q (at most 63 + 26 are read)
             const int w = (q >> 5) - 3;
             const u32 a0 = T.ring[w & 255], a1 = T.ring[(w + 1) & 255], a2 = T.ring[(w + 2) & 255], a3 = T.ring[(w + 3) & 255];
@@ -883,11 +887,20 @@ __device__ __forceinline__ bool pz_sequences(const ZArgs &A, ZBlk &b, u64 base, 
             q -= (int)((all & 31) + extra);
             // the next states' bits, LL, ML, OF from the top: shifts take a cell's low 5 bits
             const u32 head = __funnelshift_l(extra < 32 ? h1 : h0, extra < 32 ? h2 : h1, extra);
-            sl = (cl >> 21) + __funnelshift_l(head, 0u, cl);
+            sl = (cl >> 19) + 4 * __funnelshift_l(head, 0u, cl);
             const u32 h_m = __funnelshift_l(0u, head, cl);
-            sm = (cm >> 21) + __funnelshift_l(h_m, 0u, cm);
-            so = (co >> 21) + __funnelshift_l(__funnelshift_l(0u, h_m, cm), 0u, co);
+            sm = (cm >> 19) + 4 * __funnelshift_l(h_m, 0u, cm);
+            so = (co >> 19) + 4 * __funnelshift_l(__funnelshift_l(0u, h_m, cm), 0u, co);
+        };
+        if (cnt == 32) {
+#pragma unroll 8
+            for (int k = 0; k < 32; k++) step(k);
+        } else {
+            for (int k = 0; k < cnt; k++) step(k);
         }
+        my_l >>= 2;
+        my_o >>= 2;
+        my_m >>= 2;
         // after the last sequence no next states are read: their bits are not there
         if (k0 + 32 >= nseq) {
             const u32 n = (T.cell[Z_LL + my_l] + T.cell[Z_OF + my_o] + T.cell[Z_ML + my_m]) & 31;
