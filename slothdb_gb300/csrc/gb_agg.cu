@@ -570,6 +570,18 @@ static u64 next_pow2(u64 x) {
     return p;
 }
 
+// Slots of the HBM table (and of a string dictionary) for an estimated group
+// count.  A warp waits for the longest of its lanes' probe chains, a memory
+// round trip each: a small table is kept sparse (k_ingest_fast of 1M rows:
+// 1,024 groups in 2,048 slots 51 us, in 8,192 39 us; without a shared table
+// 8,192 groups in 16,384 slots 87 us, in 65,536 48 us; 4M strings of 30,000
+// into a dictionary of 65,536 slots 237 us, of 131,072 166 us), a large one a
+// quarter to half full, for its size in L2.
+static u64 table_cap(u64 est) {
+    const u64 f = est <= (1u << 13) ? 8 : (est <= (1u << 16) ? 4 : 2);
+    return std::max<u64>(1024, next_pow2(est * f));
+}
+
 struct DevBuf {
     void *p = nullptr;
     size_t n = 0;
@@ -873,9 +885,8 @@ static gb_status grow_and_merge(gb_agg *h, u64 new_cap, u32 pending, cudaStream_
             new_cap = h->cap * 2;
             continue;
         }
-        // merge [0, pending) — re-spills land at [pending, ...)
+        // merge [0, pending) — re-spills land behind what the rehash spilled at [pending, ...)
         TableRef T = table_ref(h);
-        GB_CUDA(cudaMemcpyAsync(&dctl->spill_count, &pending, sizeof(u32), cudaMemcpyHostToDevice, st));
         k_merge_records<<<grid_for(pending, 256, sm_count() * 8), 256, 0, st>>>(h->plan, (const u64 *)h->spill.p,
                                                                               pending, T);
         h->launches++;
@@ -973,10 +984,11 @@ static gb_status dist_clear(gb_agg *h, cudaStream_t st) {
     return GB_OK;
 }
 
-// defined with the fast tile path (gb_batch.cuh): launches the
-// single-query fast ingest when the plan allows it (*launched = true)
-static gb_status launch_ingest_fast(gb_agg *h, const TableRef &T, IngestArgs A, int grid, cudaStream_t st,
-                                    bool *launched);
+// defined with the fast tile path (gb_batch.cuh): whether the plan takes the
+// single-query fast ingest, and its launch
+static bool fast_ingest_plan(gb_agg *h, FastIngest &X);
+static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableRef &T, IngestArgs A, int grid,
+                                    cudaStream_t st);
 
 static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
     if (n_rows == 0) return GB_OK;
@@ -995,6 +1007,15 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
         tr = ((tr + 511) / 512) * 512;
         tile_rows = (u32)std::max<u64>(1024, std::min<u64>(tr, h->tile_rows));
     }
+    FastIngest X;
+    const bool fast = fast_ingest_plan(h, X);
+    if (fast) {
+        // as many tiles for each CTA (one, where that is under tile_rows: a CTA's row loop starts anew with each), but
+        // none of fewer than 1,024 rows
+        const u64 each = (n_rows + (u64)max_ctas * h->tile_rows - 1) / ((u64)max_ctas * h->tile_rows);
+        const u64 tr = (n_rows + max_ctas * each - 1) / (max_ctas * each);
+        tile_rows = (u32)std::max<u64>(1024, (tr + 511) / 512 * 512);
+    }
     const u64 n_tiles_total = (n_rows + tile_rows - 1) / tile_rows;
     int grid = (int)std::min<u64>((u64)max_ctas, n_tiles_total);
     // the shared table pays when the estimated groups fit it; past that every
@@ -1003,7 +1024,7 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
     if (h->est_groups > (u64)S) S = 0;
     size_t smem = (size_t)S * 8 * (1 + words);
     // spill capacity: threshold + what in-flight tiles and the final flush can add
-    u64 margin = (u64)grid * ((u64)tile_rows + (u64)S) + 1024;
+    u64 margin = (u64)grid * (2 * (u64)tile_rows + (u64)S) + 1024;
     u64 need_cap = (1u << 20) + margin;
     if (h->spill_cap < need_cap) {
         gb_status s = h->spill.ensure((size_t)need_cap * (1 + words) * 8);
@@ -1030,9 +1051,9 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
         A.pad = 0;
         TableRef T = table_ref(h);
         int g = (int)std::min<u64>((u64)grid, n_tiles_total - first);
-        bool fast = false;
-        if (gb_status fs = launch_ingest_fast(h, T, A, g, st, &fast)) return fs;
-        if (!fast) {
+        if (fast) {
+            if (gb_status fs = launch_ingest_fast(h, X, T, A, g, st)) return fs;
+        } else {
             ProfScope ps(h, "k_ingest", st);
             if (h->precombine) k_ingest<true><<<g, h->block, smem, st>>>(h->plan, T, A);
             else k_ingest<false><<<g, h->block, smem, st>>>(h->plan, T, A);
@@ -1375,9 +1396,7 @@ static gb_status strdict_encode(gb_agg *h, const uint8_t *bytes, const int64_t *
                                 const uint64_t *valid, u64 n, u64 batch_bytes, cudaStream_t st) {
     gb_status s;
     if (!h->sd_cap) {
-        u64 cap = 1024;
-        while (cap < 2 * std::max<u64>(h->est_groups, 512)) cap <<= 1;
-        if ((s = strdict_init(h, cap, st))) return s;
+        if ((s = strdict_init(h, table_cap(h->est_groups), st))) return s;
     }
     // the arena can take every string of this batch
     u64 used = 0;
@@ -1872,7 +1891,7 @@ gb_status gb_agg_estimate_bytes(const gb_agg_spec *spec, uint64_t nrows, uint64_
     if (s) return s;
     const u64 est = std::max<u64>(1, std::min<u64>(spec->est_groups ? spec->est_groups : (1u << 15),
                                                    std::max<u64>(nrows, 1)));
-    const u64 cap = std::max<u64>(1024, next_pow2(est * 2));
+    const u64 cap = table_cap(est);
     u64 b = (cap + 2) * (u64)h.plan.stride * 8;                        // hash table
     for (int t : h.out_types) b += (cap + 2) * (u64)(t == GB_T_VARCHAR ? 8 : type_size(t)) + (cap + 2) / 8;
     b += (u64)((1u << 16) + 4096) * (1 + h.plan.words) * 8;            // spill records
@@ -1937,7 +1956,7 @@ gb_status gb_agg_create(const gb_agg_spec *spec, gb_agg **out) {
     }
     gb_apply_tuning(h);
     u64 est = h->est_groups ? h->est_groups : (1u << 15);
-    h->cap = h->mode == 1 ? 4096 : std::max<u64>(1024, next_pow2(est * 2));
+    h->cap = h->mode == 1 ? 4096 : table_cap(est);
     if ((s = h->ctl_buf.ensure(sizeof(Ctl)))) {
         delete h;
         return s;
@@ -2342,7 +2361,7 @@ gb_status gb_agg_set_option(gb_agg *h, const char *name, int64_t value) {
         }
         if (h->mode != old_mode) {
             u64 est = h->est_groups ? h->est_groups : (1u << 15);
-            h->cap = h->mode == 1 ? 4096 : std::max<u64>(1024, next_pow2(est * 2));
+            h->cap = h->mode == 1 ? 4096 : table_cap(est);
             gb_status s = init_table(h, h->table, h->cap, 0);
             if (s) return s;
             GB_CUDA(cudaDeviceSynchronize());

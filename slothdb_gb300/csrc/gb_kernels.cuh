@@ -234,6 +234,18 @@ __device__ __forceinline__ long long g_slot(const TableRef &T, u64 pk, u64 h, u3
     return -1;
 }
 
+// As g_slot from its probe p0 on, by compare-and-swap at once: one round trip
+// a probe, for keys that are most often not in the table yet.
+__device__ __forceinline__ long long g_claim(const TableRef &T, u64 pk, u64 home, int p0, u32 *new_groups) {
+    for (int p = p0; p < T.gmax_probe; p++) {
+        const u64 s = (home + (u64)p) & (T.cap - 1);
+        const u64 old = atomicCAS(T.slots + s * (u64)T.stride, EMPTY_KEY, pk);
+        if (old == EMPTY_KEY) atomicAdd(new_groups, 1u);
+        if (old == EMPTY_KEY || old == pk) return (long long)s;
+    }
+    return -1;
+}
+
 __device__ __forceinline__ void apply_state(const Plan &P, u64 *w, u64 cnt, const u64 *v) {
     if (cnt) atomicAdd(w, cnt);
 #pragma unroll
@@ -511,5 +523,42 @@ __device__ __forceinline__ u64 warp_out_slot(Ctl *ctl, bool occ, unsigned active
     base = __shfl_sync(active, base, leader);
     return (u64)base + __popc(m & ((1u << lane) - 1u));
 }
+
+// ------------------------------------------------------ register-resident plans
+#define FAST_MAX_OPS 4        // ops a register-resident plan holds (single-query kernels)
+#define BATCH_FAST_MAX_OPS 2  // ops of the batch's fast plan classes
+#define FAST_MAX_FILTERS 2
+
+// Integer-plan description kept in registers by the fast tile path (up to
+// FAST_MAX_FILTERS predicates on integer or DOUBLE columns; keys SINGLE /
+// PACKED / STRING; ops ADD_I, MIN_I, MAX_I, CNT_NN over integer columns).  kdesc = key_mode | kt0 << 4 | kt1 << 8 | bits_b << 16 |
+// bits_a << 24; op[i] = kind | type << 4 | table word << 8 | shared word << 16
+// | wide << 24, wide = a MIN/MAX over BIGINT (64-bit shared word).
+struct FastPlan {
+    const void *kp[2];
+    const uint64_t *kv[2];
+    const void *vp[FAST_MAX_OPS];
+    const uint64_t *vv[FAST_MAX_OPS];
+    u32 kdesc;
+    u32 op[FAST_MAX_OPS];
+    int32_t n_filters;
+    int32_t n_ops;
+    int32_t swords;    // 32-bit words per shared state: count, then the ops
+    int32_t eligible;
+    int32_t nulls;     // some key, op or filter column has a validity mask
+};
+
+// Predicates of the fast path (read from shared memory, once per row).
+struct FastFilters {
+    const void *fp[FAST_MAX_FILTERS];
+    const uint64_t *fv[FAST_MAX_FILTERS];
+    u64 fk[FAST_MAX_FILTERS];     // constant: int64, or the bits of a double
+    u32 fdesc[FAST_MAX_FILTERS];  // column type | gb_cmp << 4
+};
+
+struct FastIngest {
+    FastPlan F;
+    FastFilters FF;
+};
 
 }  // namespace gb
