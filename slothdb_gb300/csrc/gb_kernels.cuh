@@ -30,7 +30,24 @@ struct Ctl {
     u32 err;           // ErrFlag bits
     u32 out_count;     // rows written by compaction
     u32 aux0, aux1;
+    u32 done;          // blocks of the running kernel that are through (ctl_publish)
 };
+
+// The last block of a kernel to come here writes the control words to page-
+// locked host memory: no copy of its own after the kernel (2.5 us less a call).
+// Thread 0 of every block calls it after a barrier behind the block's last
+// update.  Not for the ingest kernels: a fence behind their atomics made 10M
+// pair-key rows 415 us instead of 335.
+__device__ __forceinline__ void ctl_publish(Ctl *ctl, Ctl *host) {
+    __threadfence();
+    if (atomicAdd(&ctl->done, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const volatile u32 *from = (const volatile u32 *)ctl;
+    volatile u32 *to = (volatile u32 *)host;
+    for (u32 i = 0; i < sizeof(Ctl) / 4; i++) to[i] = from[i];
+    ctl->done = 0;
+    __threadfence_system();
+}
 
 struct TableRef {
     u64 *slots;        // (cap + 2) * stride words
