@@ -148,23 +148,28 @@ __device__ __forceinline__ i64 fast_load(const void *p, int t, u64 r) {
     }
 }
 
+// FLT: the plan may have DOUBLE ops (kernels of their own: with them the
+// integer plans' kernels were 10-20% slower).
+template <bool FLT>
 __device__ __forceinline__ u64 fast_ident(int kind) {
-    return kind == OP_MIN_I ? 0x7fffffffffffffffull : (kind == OP_MAX_I ? 0x8000000000000000ull : 0ull);
+    return kind == OP_MIN_I || (FLT && kind == OP_MIN_F)
+               ? 0x7fffffffffffffffull
+               : (kind == OP_MAX_I || (FLT && kind == OP_MAX_F) ? 0x8000000000000000ull : 0ull);
 }
 
 // Fold a partial into an HBM state (count at word 0, op i at its word).
-template <int NOPS>
+template <int NOPS, bool FLT>
 __device__ __forceinline__ void fast_apply_global(const FastPlan &F, u64 *w, u64 cnt, const u64 *v) {
     if (cnt) atomicAdd(w, cnt);
 #pragma unroll
     for (int i = 0; i < NOPS; i++) {
         const u32 od = F.op[i];
         const int kind = od & 15;
-        op_apply(kind, w + ((od >> 8) & 255), v[i], fast_ident(kind));
+        op_apply(kind, w + ((od >> 8) & 255), v[i], fast_ident<FLT>(kind));
     }
 }
 
-template <int NOPS>
+template <int NOPS, bool FLT>
 __device__ __forceinline__ void fast_global(const FastPlan &F, const TableRef &T, u64 pk, u64 cnt, const u64 *v,
                                             u32 *new_groups) {
     const long long s = g_slot(T, pk, mix64(pk), new_groups);
@@ -172,13 +177,13 @@ __device__ __forceinline__ void fast_global(const FastPlan &F, const TableRef &T
         atomicAdd(&T.ctl->spill_count, 1u);  // the query re-runs on its own handle
         return;
     }
-    fast_apply_global<NOPS>(F, T.slots + (u64)s * (u64)T.stride + 1, cnt, v);
+    fast_apply_global<NOPS, FLT>(F, T.slots + (u64)s * (u64)T.stride + 1, cnt, v);
 }
 
 // As fast_global, for the single-query kernel: a key that finds no slot
 // within the probe bound becomes a spill record (the host grows the table and
 // merges the records) instead of a re-run.
-template <int NOPS>
+template <int NOPS, bool FLT>
 __device__ __forceinline__ void fast_global_spill(const FastPlan &F, const Plan &P, const TableRef &T, u64 pk, u64 cnt,
                                                   const u64 *v, u32 *new_groups) {
     const long long s = g_slot(T, pk, mix64(pk), new_groups);
@@ -186,20 +191,21 @@ __device__ __forceinline__ void fast_global_spill(const FastPlan &F, const Plan 
         spill_record(P, T, pk, cnt, v);
         return;
     }
-    fast_apply_global<NOPS>(F, T.slots + (u64)s * (u64)T.stride + 1, cnt, v);
+    fast_apply_global<NOPS, FLT>(F, T.slots + (u64)s * (u64)T.stride + 1, cnt, v);
 }
 
 // Narrow shared states: count u32; ADD as a (lo, hi) u32 pair with carry;
-// CNT_NN u32; MIN/MAX s32 over SMALLINT/INTEGER, s64 over BIGINT.  Every
-// update is a native 32-bit shared atomic except the 64-bit MIN/MAX.
-template <int NOPS>
+// CNT_NN u32; MIN/MAX s32 over SMALLINT/INTEGER, s64 over BIGINT and (order
+// preserving) DOUBLE; a DOUBLE sum is a double.  Every update is a native
+// 32-bit shared atomic except the 64-bit MIN/MAX and the DOUBLE sum.
+template <int NOPS, bool FLT>
 __device__ __forceinline__ void fast_apply_smem(const FastPlan &F, u32 *st, u64 cnt, const u64 *v) {
     atomicAdd(st, (u32)cnt);
 #pragma unroll
     for (int i = 0; i < NOPS; i++) {
         const u32 od = F.op[i];
         const int kind = od & 15;
-        if (v[i] == fast_ident(kind)) continue;
+        if (v[i] == fast_ident<FLT>(kind)) continue;
         u32 *w = st + ((od >> 16) & 255);
         const bool wide = (od >> 24) & 1;
         switch (kind) {
@@ -218,8 +224,11 @@ __device__ __forceinline__ void fast_apply_smem(const FastPlan &F, u32 *st, u64 
             if (wide) atomicMax((long long *)w, (long long)v[i]);
             else atomicMax((int *)w, (int)(i64)v[i]);
             break;
-        default:  // CNT_NN
-            atomicAdd(w, (u32)v[i]);
+        default:  // CNT_NN, the DOUBLE ops
+            if (!FLT || kind == OP_CNT_NN) atomicAdd(w, (u32)v[i]);
+            else if (kind == OP_ADD_F) atomicAdd((double *)w, __longlong_as_double((i64)v[i]));
+            else if (kind == OP_MIN_F) atomicMin((long long *)w, (long long)v[i]);
+            else atomicMax((long long *)w, (long long)v[i]);
             break;
         }
     }
@@ -232,10 +241,14 @@ __device__ __forceinline__ u32 smem_hash(u64 pk, int S) {
     return (x >> 16) * (u32)S >> 16;
 }
 
-template <int NOPS>
+// Two states follow the table's, for the rows whose key is NULL or the empty
+// marker: their groups' out-of-band HBM slots take one fold per CTA (3M rows,
+// 5% NULL keys, 64 groups, DOUBLE sum: 201 us with a fold a row into one slot,
+// 65 us).
+template <int NOPS, bool FLT>
 __device__ __forceinline__ void fast_smem_init(const FastPlan &F, u64 *keys, u32 *st, int S) {
-    for (int i = threadIdx.x; i < S; i += blockDim.x) {
-        keys[i] = EMPTY_KEY;
+    for (int i = threadIdx.x; i < S + 2; i += blockDim.x) {
+        if (i < S) keys[i] = EMPTY_KEY;
         u32 *w = st + (u64)i * F.swords;
         w[0] = 0;
 #pragma unroll
@@ -244,12 +257,13 @@ __device__ __forceinline__ void fast_smem_init(const FastPlan &F, u64 *keys, u32
             const int kind = od & 15;
             u32 *x = w + ((od >> 16) & 255);
             const bool wide = (od >> 24) & 1;
-            if (kind == OP_ADD_I) {
+            if (wide) {
+                *(u64 *)x = fast_ident<FLT>(kind);
+            } else if (kind == OP_ADD_I) {
                 x[0] = 0;
                 x[1] = 0;
             } else if (kind == OP_MIN_I || kind == OP_MAX_I) {
-                if (wide) *(u64 *)x = fast_ident(kind);
-                else x[0] = kind == OP_MIN_I ? 0x7fffffffu : 0x80000000u;
+                x[0] = kind == OP_MIN_I ? 0x7fffffffu : 0x80000000u;
             } else {
                 x[0] = 0;
             }
@@ -261,11 +275,32 @@ __device__ __forceinline__ void fast_smem_init(const FastPlan &F, u64 *keys, u32
 // flight at a time, and CTAs begin at different places, as they hold much the
 // same keys (1M rows, 1,024 groups: 38.7 us; one slot at a time 40.7, all CTAs
 // in step 41.0 us).
-template <int NOPS, bool SPILL = false>
+template <int NOPS, bool FLT, bool SPILL = false>
 __device__ __forceinline__ void fast_smem_flush(const FastPlan &F, const TableRef &T, const u64 *keys, const u32 *st,
                                                 int S, u32 *new_groups, const Plan *SP = nullptr) {
     constexpr int U = 4;
     const u32 turn = blockIdx.x * 0x9e3779b1u >> 16;
+    auto state = [&](const u32 *w, u64 *v) {
+#pragma unroll
+        for (int j = 0; j < NOPS; j++) {
+            const u32 od = F.op[j];
+            const int kind = od & 15;
+            const u32 *x = w + ((od >> 16) & 255);
+            const bool wide = (od >> 24) & 1;
+            if (wide) v[j] = *(const u64 *)x;
+            else if (kind == OP_ADD_I) v[j] = (u64)x[0] | ((u64)x[1] << 32);
+            else if (kind == OP_MIN_I || kind == OP_MAX_I) v[j] = (u64)(i64)(int)x[0];
+            else v[j] = x[0];
+        }
+    };
+    if (threadIdx.x < 2) {
+        const u32 *w = st + (u64)(S + threadIdx.x) * F.swords;
+        if (w[0]) {
+            u64 v[NOPS ? NOPS : 1];
+            state(w, v);
+            fast_apply_global<NOPS, FLT>(F, T.slots + (T.cap + threadIdx.x) * (u64)T.stride + 1, w[0], v);
+        }
+    }
     for (int i0 = threadIdx.x; i0 < S; i0 += U * blockDim.x) {
         u64 k[U], g[U], at[U];
 #pragma unroll
@@ -281,19 +316,10 @@ __device__ __forceinline__ void fast_smem_flush(const FastPlan &F, const TableRe
             if (k[u] == EMPTY_KEY) continue;
             const u32 *w = st + (u64)(((u32)(i0 + u * blockDim.x) + turn) & (u32)(S - 1)) * F.swords;
             u64 v[NOPS ? NOPS : 1];
-#pragma unroll
-            for (int j = 0; j < NOPS; j++) {
-                const u32 od = F.op[j];
-                const int kind = od & 15;
-                const u32 *x = w + ((od >> 16) & 255);
-                const bool wide = (od >> 24) & 1;
-                if (kind == OP_ADD_I) v[j] = (u64)x[0] | ((u64)x[1] << 32);
-                else if (kind == OP_MIN_I || kind == OP_MAX_I) v[j] = wide ? *(const u64 *)x : (u64)(i64)(int)x[0];
-                else v[j] = x[0];
-            }
+            state(w, v);
             long long s = (long long)at[u];
             if (g[u] != k[u]) s = g_claim(T, k[u], at[u], g[u] == EMPTY_KEY ? 0 : 1, new_groups);
-            if (s >= 0) fast_apply_global<NOPS>(F, T.slots + (u64)s * (u64)T.stride + 1, w[0], v);
+            if (s >= 0) fast_apply_global<NOPS, FLT>(F, T.slots + (u64)s * (u64)T.stride + 1, w[0], v);
             else if (SPILL) spill_record(*SP, T, k[u], w[0], v);
             else atomicAdd(&T.ctl->spill_count, 1u);  // the query re-runs on its own handle
         }
@@ -383,7 +409,7 @@ __device__ __forceinline__ int fast_key_of(u32 kd, i64 a_, i64 b_, u32 vbits, u6
 }
 
 // One warp step of the fast path on fetched rows.
-template <bool PRECOMBINE, int NOPS, bool FILT, bool SPILL = false>
+template <bool PRECOMBINE, int NOPS, bool FILT, bool FLT, bool SPILL = false>
 __device__ __forceinline__ void fast_rows(const FastPlan &F, const FastFilters &FF, const TableRef &T, u64 *keys,
                                           u32 *st, int S, const FastRaw<NOPS, FILT> &w, u32 *new_groups,
                                           const Plan *SP = nullptr) {
@@ -394,13 +420,15 @@ __device__ __forceinline__ void fast_rows(const FastPlan &F, const FastFilters &
 #pragma unroll
     for (int i = 0; i < NOPS; i++) {
         const int kind = F.op[i] & 15;
-        v[i] = fast_ident(kind);
+        v[i] = fast_ident<FLT>(kind);
         if (act && (w.vbits & (4u << i))) v[i] = kind == OP_CNT_NN ? 1ull : (u64)w.x[i];
+        if (FLT && (kind == OP_MIN_F || kind == OP_MAX_F) && act && (w.vbits & (4u << i)))
+            v[i] = (u64)enc_f64(__longlong_as_double(w.x[i]));
     }
     if (act) {
         const int kind = fast_key_of(F.kdesc, w.a, w.b, w.vbits, pk);
         if (kind != 0) {
-            fast_apply_global<NOPS>(F, T.slots + (T.cap + (u64)(kind - 1)) * (u64)T.stride + 1, 1, v);
+            fast_apply_smem<NOPS, FLT>(F, st + (u64)(S + kind - 1) * F.swords, 1, v);
             act = false;
         }
     }
@@ -444,12 +472,12 @@ __device__ __forceinline__ void fast_rows(const FastPlan &F, const FastFilters &
             }
             if (!__any_sync(FULL, open)) break;
         }
-        if (act && !open) fast_apply_smem<NOPS>(F, st + (u64)s * F.swords, cnt, v);
+        if (act && !open) fast_apply_smem<NOPS, FLT>(F, st + (u64)s * F.swords, cnt, v);
         act = open;
     }
     if (!act) return;
-    if (SPILL) fast_global_spill<NOPS>(F, *SP, T, pk, cnt, v, new_groups);
-    else fast_global<NOPS>(F, T, pk, cnt, v, new_groups);
+    if (SPILL) fast_global_spill<NOPS, FLT>(F, *SP, T, pk, cnt, v, new_groups);
+    else fast_global<NOPS, FLT>(F, T, pk, cnt, v, new_groups);
 }
 
 // One tile of the fast path (inlined into its class's kernel: the plan's
@@ -458,10 +486,10 @@ template <bool PRECOMBINE, int NOPS, bool NULLS, bool FILT>
 __device__ __forceinline__ void fast_tile(const FastPlan &F, const FastFilters &FF, const TableRef &T, u64 *bsm,
                                           int smem_bytes, int S, u64 t0, u64 t1, u32 *new_groups) {
     const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    while (S && (size_t)S * (8 + 4 * (size_t)F.swords) > (size_t)smem_bytes) S >>= 1;
+    while (S && FAST_SMEM(S, F.swords) > (size_t)smem_bytes) S >>= 1;
     u64 *keys = bsm;
     u32 *st = (u32 *)(bsm + S);
-    fast_smem_init<NOPS>(F, keys, st, S);
+    fast_smem_init<NOPS, false>(F, keys, st, S);
     __syncthreads();
     const u64 step = (u64)nwarps * 32;
     u64 base = t0 + (u64)warp * 32;
@@ -469,11 +497,11 @@ __device__ __forceinline__ void fast_tile(const FastPlan &F, const FastFilters &
     fast_fetch<NOPS, NULLS, FILT>(F, FF, base + (threadIdx.x & 31), t1, cur);
     for (; base < t1; base += step) {
         fast_fetch<NOPS, NULLS, FILT>(F, FF, base + step + (threadIdx.x & 31), t1, nxt);
-        fast_rows<PRECOMBINE, NOPS, FILT>(F, FF, T, keys, st, S, cur, new_groups);
+        fast_rows<PRECOMBINE, NOPS, FILT, false>(F, FF, T, keys, st, S, cur, new_groups);
         cur = nxt;
     }
     __syncthreads();
-    fast_smem_flush<NOPS>(F, T, keys, st, S, new_groups);
+    fast_smem_flush<NOPS, false>(F, T, keys, st, S, new_groups);
 }
 
 // One tile of the generic path (any plan; the plan is in shared memory).
@@ -817,7 +845,7 @@ struct gb_batch {
 
 // The fast-path description of a query's plan (eligible = 0 when the plan
 // has more than FAST_MAX_FILTERS predicates or an IN / VARCHAR predicate, a
-// full-width pair key, floating-point ops or more than max_ops ops: such
+// full-width pair key, COUNT(DISTINCT) or more than max_ops ops: such
 // queries take the generic tile path).
 static FastPlan make_fast_plan(const Plan &P, FastFilters &FF, int max_ops = BATCH_FAST_MAX_OPS) {
     FastPlan F;
@@ -841,9 +869,12 @@ static FastPlan make_fast_plan(const Plan &P, FastFilters &FF, int max_ops = BAT
     for (int i = 0; i < P.n_ops; i++) {
         const Op &o = P.ops[i];
         const int t = P.cols[o.col].type;
-        if (o.kind != OP_ADD_I && o.kind != OP_MIN_I && o.kind != OP_MAX_I && o.kind != OP_CNT_NN) return F;
-        if (o.kind != OP_CNT_NN && !is_int(t)) return F;
-        const bool wide = (o.kind == OP_MIN_I || o.kind == OP_MAX_I) && t == GB_T_BIGINT;
+        if (o.kind == OP_DIST || o.kind == OP_NONE) return F;
+        const bool flt = o.kind == OP_ADD_F || o.kind == OP_MIN_F || o.kind == OP_MAX_F;
+        if (o.kind != OP_CNT_NN && !(flt ? t == GB_T_DOUBLE : is_int(t))) return F;
+        const bool wide = flt || ((o.kind == OP_MIN_I || o.kind == OP_MAX_I) && t == GB_T_BIGINT);
+        F.flt |= flt;
+        F.sums_f |= o.kind == OP_ADD_F;
         if (wide && (sw & 1)) sw++;
         F.op[i] = (u32)o.kind | ((u32)(t & 15) << 4) | ((u32)o.word << 8) | ((u32)sw << 16) | ((u32)wide << 24);
         sw += (wide || o.kind == OP_ADD_I) ? 2 : 1;
@@ -878,7 +909,7 @@ static FastPlan make_fast_plan(const Plan &P, FastFilters &FF, int max_ops = BAT
 // query's tiles, with one narrow shared table per CTA for the whole launch
 // and spill records instead of re-runs.  Same tile-claim / spill-threshold
 // protocol as k_ingest, so run_ingest drives both.
-template <bool PRE, int NOPS, bool NULLS, bool FILT>
+template <bool PRE, int NOPS, bool NULLS, bool FILT, bool FLT = false>
 __global__ void __launch_bounds__(512, 2)
     k_ingest_fast(const __grid_constant__ Plan P, const __grid_constant__ FastPlan F,
                   const __grid_constant__ FastFilters FF, const TableRef T, const IngestArgs A) {
@@ -894,7 +925,7 @@ __global__ void __launch_bounds__(512, 2)
         s_tile[to] = t;
     };
     if (threadIdx.x == 0) claim(0);
-    fast_smem_init<NOPS>(F, keys, st, S);
+    fast_smem_init<NOPS, FLT>(F, keys, st, S);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 step = (u64)(blockDim.x >> 5) * 32;
@@ -909,7 +940,7 @@ __global__ void __launch_bounds__(512, 2)
         fast_fetch<NOPS, NULLS, FILT>(F, FF, base + lane, t1, cur);
         for (; base < t1; base += step) {
             fast_fetch<NOPS, NULLS, FILT>(F, FF, base + step + lane, t1, nxt);
-            fast_rows<PRE, NOPS, FILT, true>(F, FF, T, keys, st, S, cur, &s_new, &P);
+            fast_rows<PRE, NOPS, FILT, FLT, true>(F, FF, T, keys, st, S, cur, &s_new, &P);
             cur = nxt;
         }
         if (threadIdx.x == 0 && *(volatile u32 *)&T.ctl->spill_count > T.spill_threshold)
@@ -917,7 +948,7 @@ __global__ void __launch_bounds__(512, 2)
         __syncthreads();
     }
     __syncthreads();
-    fast_smem_flush<NOPS, true>(F, T, keys, st, S, &s_new, &P);
+    fast_smem_flush<NOPS, FLT, true>(F, T, keys, st, S, &s_new, &P);
     __syncthreads();
     if (threadIdx.x == 0 && s_new) atomicAdd(&T.ctl->n_groups, s_new);
 }
@@ -931,6 +962,18 @@ typedef void (*FastIngestKernel)(Plan, FastPlan, FastFilters, TableRef, IngestAr
             k_ingest_fast<PRE_, N_, true, false>, k_ingest_fast<PRE_, N_, true, true>           \
         }                                                                                       \
     }
+
+// Plans with DOUBLE ops: one kernel for each number of ops, with the NULL and
+// predicate code whether they need it or not.
+static FastIngestKernel fast_ingest_kernel_f(int pre, int nops) {
+    static const FastIngestKernel tab[2][FAST_MAX_OPS] = {
+        {k_ingest_fast<false, 1, true, true, true>, k_ingest_fast<false, 2, true, true, true>,
+         k_ingest_fast<false, 3, true, true, true>, k_ingest_fast<false, 4, true, true, true>},
+        {k_ingest_fast<true, 1, true, true, true>, k_ingest_fast<true, 2, true, true, true>,
+         k_ingest_fast<true, 3, true, true, true>, k_ingest_fast<true, 4, true, true, true>},
+    };
+    return tab[pre][nops - 1];
+}
 
 static FastIngestKernel fast_ingest_kernel(int pre, int nops, int nulls, int filt) {
     static const FastIngestKernel tab[2][FAST_MAX_OPS + 1][2][2] = {
@@ -955,9 +998,10 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
     const int S = h->est_groups <= (u64)A.smem_slots ? A.smem_slots : 0;
     // narrow shared atomics beat the warp key match; without a shared table,
     // few groups mean hot HBM slots, which the match relieves
-    const bool pre = h->precombine_set ? h->precombine : (S == 0 && h->est_groups <= 4096);
+    const bool pre = h->precombine_set ? h->precombine
+                                       : (S == 0 ? h->est_groups <= 4096 : F.sums_f && h->est_groups <= FAST_PRE_F);
     A.smem_slots = S;
-    const size_t smem = (size_t)S * (8 + 4 * (size_t)F.swords);
+    const size_t smem = FAST_SMEM(S, F.swords);
     static bool attr_set = false;
     if (!attr_set) {
         for (int a = 0; a < 2; a++)
@@ -966,12 +1010,17 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
                     for (int f = 0; f < 2; f++)
                         GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel(a, n, u, f),
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        for (int a = 0; a < 2; a++)
+            for (int n = 1; n <= FAST_MAX_OPS; n++)
+                GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel_f(a, n), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             200 * 1024));
         attr_set = true;
     }
     {
         ProfScope ps(h, "k_ingest_fast", st);
-        fast_ingest_kernel(pre, F.n_ops, F.nulls != 0, F.n_filters != 0)<<<grid, 512, smem, st>>>(h->plan, F, X.FF,
-                                                                                                   T, A);
+        const FastIngestKernel k = F.flt ? fast_ingest_kernel_f(pre, F.n_ops)
+                                         : fast_ingest_kernel(pre, F.n_ops, F.nulls != 0, F.n_filters != 0);
+        k<<<grid, 512, smem, st>>>(h->plan, F, X.FF, T, A);
     }
     GB_CUDA(cudaGetLastError());
     return GB_OK;
@@ -982,7 +1031,7 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
 static int batch_smem_bytes(int ctas) {
     int b = (227 * 1024) / std::max(1, ctas) - 4096;
     b = std::min(b, 96 * 1024);
-    return b & ~4095;
+    return (b & ~4095) + 256;  // the fast path's out-of-band states beside a table of a power of two slots
 }
 
 static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
@@ -1047,6 +1096,7 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
         }
         d.P = h->plan;
         if (b->fast) d.F = make_fast_plan(h->plan, d.FF);
+        if (d.F.flt) d.F.eligible = 0;  // DOUBLE ops: the generic tiles
         d.T = table_ref(h);
         d.T.ctl = (Ctl *)b->qctl.p + q;
         d.T.spill_threshold = h->spill_cap / 2;
@@ -1056,9 +1106,8 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
         if (d.F.eligible) {
             // narrow shared states: as many slots as fit, used when the
             // estimated groups fit in them (else rows go straight to HBM)
-            const int per = 8 + 4 * d.F.swords;
             int S = 1;
-            while (S * 2 * per <= batch_smem_bytes(b->ctas_per_sm)) S *= 2;
+            while (FAST_SMEM(S * 2, d.F.swords) <= (size_t)batch_smem_bytes(b->ctas_per_sm)) S *= 2;
             S = std::min(S, b->smem_slots_max);
             d.smem_slots = h->est_groups <= (u64)S ? S : 0;
             // narrow shared atomics beat the warp key match; without a shared
@@ -1156,7 +1205,7 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {
         for (int c = 0; c < BATCH_CLASSES; c++)
-            cudaFuncSetAttribute(batch_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+            cudaFuncSetAttribute(batch_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024 + 256);
         attr = true;
     }
     b->prepared = true;

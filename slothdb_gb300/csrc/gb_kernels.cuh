@@ -545,12 +545,18 @@ __device__ __forceinline__ u64 warp_out_slot(Ctl *ctl, bool occ, unsigned active
 #define FAST_MAX_OPS 4        // ops a register-resident plan holds (single-query kernels)
 #define BATCH_FAST_MAX_OPS 2  // ops of the batch's fast plan classes
 #define FAST_MAX_FILTERS 2
+// shared memory of a CTA's table of S slots: keys, states, two out-of-band states
+#define FAST_SMEM(S, swords) ((size_t)(S) * 8 + ((size_t)(S) + 2) * 4 * (size_t)(swords))
+// with a DOUBLE sum in shared memory (a compare-and-swap loop), a warp's equal
+// keys are combined first for up to so many estimated groups (3M rows: 3
+// groups 106 us with, 303 without; 64 groups 77 and 65 us)
+#define FAST_PRE_F 24
 
-// Integer-plan description kept in registers by the fast tile path (up to
+// Plan description kept in registers by the fast tile path (up to
 // FAST_MAX_FILTERS predicates on integer or DOUBLE columns; keys SINGLE /
-// PACKED / STRING; ops ADD_I, MIN_I, MAX_I, CNT_NN over integer columns).  kdesc = key_mode | kt0 << 4 | kt1 << 8 | bits_b << 16 |
+// PACKED / STRING; any ops but OP_DIST).  kdesc = key_mode | kt0 << 4 | kt1 << 8 | bits_b << 16 |
 // bits_a << 24; op[i] = kind | type << 4 | table word << 8 | shared word << 16
-// | wide << 24, wide = a MIN/MAX over BIGINT (64-bit shared word).
+// | wide << 24, wide = a 64-bit shared word (MIN/MAX over BIGINT, the DOUBLE ops).
 struct FastPlan {
     const void *kp[2];
     const uint64_t *kv[2];
@@ -563,6 +569,8 @@ struct FastPlan {
     int32_t swords;    // 32-bit words per shared state: count, then the ops
     int32_t eligible;
     int32_t nulls;     // some key, op or filter column has a validity mask
+    int32_t flt;       // some op is over DOUBLE
+    int32_t sums_f;    // some op is a DOUBLE sum
 };
 
 // Predicates of the fast path (read from shared memory, once per row).

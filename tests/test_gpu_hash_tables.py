@@ -62,3 +62,25 @@ def test_keys_of_one_residue(spread):
     s = rng.integers(-100, 100, len(k)).astype(np.int16)
     types = [BIGINT, BIGINT, SMALLINT]
     compare(run(types, [0], AGGS, [k, v, s], 1500), oracle.run_query(types, [0], AGGS, [k, v, s]))
+
+
+@pytest.mark.parametrize("groups", [1, 20, 30, 1000, 3000, 60_000])
+@pytest.mark.parametrize("filtered", [False, True])
+def test_double_ops_and_null_keys(groups, filtered):
+    """DOUBLE SUM / AVG / MIN / MAX beside counts, with NULL keys and values
+    and the INT64_MIN key, in shared and HBM tables and through the warp's key
+    match."""
+    n = 60_011 + groups
+    rng = np.random.default_rng(groups)
+    k = rng.integers(0, groups, n)
+    k[::977] = np.iinfo(np.int64).min
+    x = rng.normal(100, 25, n)
+    f = rng.integers(0, 1000, n).astype(np.int16)
+    nulls = [rng.random(n) < 0.1, rng.random(n) < 0.07, None]
+    types = [BIGINT, capi.DOUBLE, SMALLINT]
+    aggs = [("count_star", -1), ("sum", 1), ("avg", 1), ("min", 1), ("max", 1)]
+    filters = [(2, "<", 700)] if filtered else []
+    cols = [k, x, f]
+    orc = oracle.run_query(types, [0], aggs, cols, filters=filters, nulls=nulls)
+    for options in (None, {"precombine": 1}):
+        compare(run(types, [0], aggs, cols, groups, filters=filters, nulls=nulls, options=options), orc)
