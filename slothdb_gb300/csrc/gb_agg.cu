@@ -55,16 +55,19 @@ struct ResetArgs {
     uint64_t *valid[2 + GB_MAX_AGGS];
 };
 
-// Bound by its writes: 16 bytes a thread and step (slots are of an even
-// number of words).  33 MB of pair-key table: 15.6 -> 14.6 us.
-__global__ void k_table_init(u64 *slots, u64 nslots, int stride, const __grid_constant__ Plan P,
+// Bound by its writes: 16 bytes a thread and step (the states, cap + 2 of them,
+// then the keys: an even number of words each).
+__global__ void k_table_init(u64 *table, u64 cap, int stride, const __grid_constant__ Plan P,
                              const __grid_constant__ ResetArgs R) {
     const u64 me = blockIdx.x * (u64)blockDim.x + threadIdx.x, all = (u64)gridDim.x * blockDim.x;
-    const u64 total = nslots * (u64)stride / 2;
-    auto word = [&](u32 w) -> u64 { return w == 0 ? EMPTY_KEY : (w <= (u32)P.words ? P.word_init[w - 1] : 0ull); };
+    const u64 states = (cap + 2) * (u64)stride / 2, total = states + cap / 2;
+    auto word = [&](u32 w) -> u64 { return w < (u32)P.words ? P.word_init[w] : 0ull; };
     for (u64 i = me; i < total; i += all) {
-        const u32 w = total < (1ull << 31) ? 2u * (u32)i % (u32)stride : (u32)(2 * i % (u64)stride);
-        *(ulonglong2 *)(slots + 2 * i) = make_ulonglong2(word(w), word(w + 1));
+        const u64 at = 2 * i;
+        const u32 w0 = total < (1ull << 30) ? (u32)at % (u32)stride : (u32)(at % (u64)stride);
+        const u32 w1 = w0 + 1 == (u32)stride ? 0 : w0 + 1;
+        *(ulonglong2 *)(table + at) =
+            i >= states ? make_ulonglong2(EMPTY_KEY, EMPTY_KEY) : make_ulonglong2(word(w0), word(w1));
     }
     if (!R.ctl) return;
     for (int c = 0; c < R.n_valid; c++)
@@ -170,22 +173,22 @@ __global__ void k_rehash(const __grid_constant__ Plan P, const u64 *old, u64 old
     for (u64 s = blockIdx.x * (u64)blockDim.x + threadIdx.x; s < old_cap + 2; s += (u64)gridDim.x * blockDim.x) {
         const u64 *src = old + s * (u64)stride;
         if (s >= old_cap) {
-            if (src[1] == 0) continue;
-            u64 *dst = T.slots + (T.cap + (s - old_cap)) * (u64)T.stride;
-            for (int w = 0; w < P.words; w++) dst[1 + w] = src[1 + w];
+            if (src[0] == 0) continue;
+            u64 *dst = T.states + (T.cap + (s - old_cap)) * (u64)T.stride;
+            for (int w = 0; w < P.words; w++) dst[w] = src[w];
             continue;
         }
-        u64 k = src[0];
+        const u64 k = old[(old_cap + 2) * (u64)stride + s];
         if (k == EMPTY_KEY) continue;
         long long d = g_slot(T, k, mix64(k), &s_new);
         if (d < 0) {
             u64 v[GB_MAX_OPS];
-            for (int i = 0; i < P.n_ops; i++) v[i] = src[1 + P.ops[i].word];
-            spill_record(P, T, k, src[1], v);
+            for (int i = 0; i < P.n_ops; i++) v[i] = src[P.ops[i].word];
+            spill_record(P, T, k, src[0], v);
             continue;
         }
-        u64 *dst = T.slots + (u64)d * (u64)T.stride;
-        for (int w = 0; w < P.words; w++) dst[1 + w] = src[1 + w];
+        u64 *dst = T.states + (u64)d * (u64)T.stride;
+        for (int w = 0; w < P.words; w++) dst[w] = src[w];
     }
     __syncthreads();
     if (threadIdx.x == 0 && s_new) atomicAdd(&T.ctl->n_groups, s_new);
@@ -213,7 +216,7 @@ __global__ void k_merge_records(const __grid_constant__ Plan P, const u64 *recs,
 // tables use fewer slots per thread so that more CTAs share them); one
 // output reservation per chunk.
 #define COMPACT_PER 8
-__global__ void k_compact(const __grid_constant__ Plan P, const u64 *slots, u64 cap, int stride,
+__global__ void k_compact(const __grid_constant__ Plan P, const u64 *keys, const u64 *states, u64 cap, int stride,
                           const __grid_constant__ EmitArgs E, Ctl *ctl, int per, Ctl *ctl_host) {
     const u64 total = cap + 2;
     const u64 chunk = (u64)per * blockDim.x;
@@ -223,23 +226,23 @@ __global__ void k_compact(const __grid_constant__ Plan P, const u64 *slots, u64 
         for (int j = 0; j < COMPACT_PER; j++) {
             const u64 s = c0 + (u64)j * blockDim.x + threadIdx.x;
             if (j >= per || s >= total) break;
-            const u64 *sl = slots + s * (u64)stride;
-            mine += (s < cap) ? (sl[0] != EMPTY_KEY) : (sl[1] != 0);
+            mine += (s < cap) ? (keys[s] != EMPTY_KEY) : (states[s * (u64)stride] != 0);
         }
         u64 o = block_out_base(ctl, mine);
 #pragma unroll
         for (int j = 0; j < COMPACT_PER; j++) {
             const u64 s = c0 + (u64)j * blockDim.x + threadIdx.x;
             if (j >= per || s >= total) break;
-            const u64 *sl = slots + s * (u64)stride;
-            const bool occ = (s < cap) ? (sl[0] != EMPTY_KEY) : (sl[1] != 0);
+            const u64 *sl = states + s * (u64)stride;
+            const u64 k = s < cap ? keys[s] : EMPTY_KEY;
+            const bool occ = (s < cap) ? (k != EMPTY_KEY) : (sl[0] != 0);
             if (!occ) continue;
             if (o >= E.out_cap) {
                 atomicOr(&ctl->err, (u32)ERR_OUT_OVERFLOW);
                 continue;
             }
-            const u64 pk = (s < cap) ? sl[0] : (s == cap ? EMPTY_KEY : 0ull);
-            emit_group(P, E, o, pk, s == cap + 1, sl + 1);
+            const u64 pk = s <= cap ? k : 0ull;
+            emit_group(P, E, o, pk, s == cap + 1, sl);
             o++;
         }
     }
@@ -615,6 +618,9 @@ static u64 table_cap(u64 est) {
     return std::max<u64>(1024, next_pow2(est * f));
 }
 
+// Words of a table: cap + 2 states, then cap keys.
+static u64 table_words(const Plan &P, u64 cap) { return (cap + 2) * (u64)P.stride + cap; }
+
 struct DevBuf {
     void *p = nullptr;
     size_t n = 0;
@@ -769,7 +775,9 @@ struct gb_agg {
 
 static TableRef table_ref(gb_agg *h) {
     TableRef T;
-    T.slots = (u64 *)h->table.p;
+    T.states = (u64 *)h->table.p;
+    T.keys = T.states + (h->cap + 2) * (u64)h->plan.stride;
+    T.kstride = 1;
     T.cap = h->cap;
     T.stride = h->plan.stride;
     T.gmax_probe = h->gmax_probe;
@@ -844,14 +852,14 @@ static int grid_for(u64 work, int block, int max_ctas) {
 static gb_status alloc_outputs(gb_agg *h, u64 rows);
 
 static gb_status init_table(gb_agg *h, DevBuf &buf, u64 cap, cudaStream_t st, const ResetArgs *reset = nullptr) {
-    size_t bytes = (size_t)(cap + 2) * h->plan.stride * 8;
+    size_t bytes = (size_t)table_words(h->plan, cap) * 8;
     gb_status s = buf.ensure(bytes);
     if (s) return s;
-    u64 words = (cap + 2) * (u64)h->plan.stride;
+    u64 words = table_words(h->plan, cap);
     {
         ProfScope ps(h, "k_table_init", st);
         const ResetArgs none{};
-        k_table_init<<<grid_for(words / 2, 256, sm_count() * 8), 256, 0, st>>>((u64 *)buf.p, cap + 2, h->plan.stride,
+        k_table_init<<<grid_for(words / 2, 256, sm_count() * 8), 256, 0, st>>>((u64 *)buf.p, cap, h->plan.stride,
                                                                                h->plan, reset ? *reset : none);
     }
     h->launches++;
@@ -1820,9 +1828,8 @@ static gb_status compile_plan(gb_agg *h) {
     }
     if (h->str_col >= 0) P.n_cols = nc + 1;
     {
-        int need = words + 1;
-        int stride = need <= 4 ? (int)next_pow2(need) : ((need + 3) / 4) * 4;
-        P.stride = stride;
+        // states of 1, 2 or 4 words, or of whole 32-byte sectors
+        P.stride = words <= 4 ? (int)next_pow2(words) : (words + 3) / 4 * 4;
     }
     return GB_OK;
 too_many:
@@ -1958,7 +1965,7 @@ gb_status gb_agg_estimate_bytes(const gb_agg_spec *spec, uint64_t nrows, uint64_
     const u64 est = std::max<u64>(1, std::min<u64>(spec->est_groups ? spec->est_groups : (1u << 15),
                                                    std::max<u64>(nrows, 1)));
     const u64 cap = table_cap(est);
-    u64 b = (cap + 2) * (u64)h.plan.stride * 8;                        // hash table
+    u64 b = table_words(h.plan, cap) * 8;                               // hash table
     for (int t : h.out_types) b += (cap + 2) * (u64)(t == GB_T_VARCHAR ? 8 : type_size(t)) + (cap + 2) / 8;
     b += (u64)((1u << 16) + 4096) * (1 + h.plan.words) * 8;            // spill records
     if (h.str_col >= 0) b += 4 * 2 * cap * 8 + 40 * est + 16 * est;    // dictionary, arena, emitted strings
@@ -2273,13 +2280,14 @@ gb_status gb_agg_finalize(gb_agg *h, void *stream) {
     fill_emit(h, E, h->out_cols, h->out_valid, h->out_cap);
     {
         ProfScope ps(h, "k_compact", st);
+        const TableRef T = table_ref(h);
         // slots per thread: up to COMPACT_PER, fewer where the table would
         // otherwise occupy under two CTAs per SM
         const u64 slots_n = h->cap + 2;
         int per = COMPACT_PER;
         while (per > 1 && slots_n / ((u64)per * 256) < (u64)sm_count() * 2) per >>= 1;
         k_compact<<<grid_for((slots_n + per - 1) / per, 256, sm_count() * 4), 256, 0, st>>>(
-            h->plan, (const u64 *)h->table.p, h->cap, h->plan.stride, E, dctl, per, (Ctl *)h->ctl_pin.p);
+            h->plan, T.keys, T.states, h->cap, h->plan.stride, E, dctl, per, (Ctl *)h->ctl_pin.p);
     }
     h->launches++;
     GB_CUDA(cudaGetLastError());

@@ -1,10 +1,13 @@
 // gb_internal.cuh — device/host internals shared by the GROUP BY kernels.
 //
-// Hash-table layout (HBM): a power-of-two array of slots, each `stride`
-// 64-bit words: word 0 = packed group key (EMPTY_KEY = free), words
-// 1..words = aggregate state words.  State word 0 is always the row count
-// of the group (COUNT(*) reads it; it also marks the two out-of-band slots
-// cap+0 = "key equals EMPTY_KEY" and cap+1 = "NULL key" as used).
+// Hash-table layout (HBM): a power-of-two number of slots in two arrays, the
+// packed group keys (one word each, EMPTY_KEY = free) and the states (`stride`
+// 64-bit words a slot).  State word 0 is always the row count of the group
+// (COUNT(*) reads it; it also marks the two out-of-band states cap+0 = "key
+// equals EMPTY_KEY" and cap+1 = "NULL key" as used).  Keys are read by every
+// row and written once, states take atomics from every row: in one line with
+// them, each atomic sent the copies of the key back to the other die's L2
+// (10M rows of 300,000 pair keys: 335 us in one array, 290 us in two).
 //
 // The per-group state is the GPU restatement of the reference's AggState
 // (src/execution/physical_planner.cpp:6080-6128): count, sum, min, max.
@@ -98,7 +101,7 @@ struct Plan {
     int32_t key_bits_b;   // KEY_PACKED: width of the second key
     int32_t key_bits_a;   // KEY_PACKED: width of the first key
     int32_t words;        // state words (word 0 = row count)
-    int32_t stride;       // words per table slot incl. key, power of two
+    int32_t stride;       // words of a slot's state
     int32_t n_dist;       // OP_DIST ops (COUNT(DISTINCT) columns)
     int32_t dnarrow;      // 1: pair sets of 8-byte slots (a non-NULL 16/32-bit key, 16/32-bit values)
     int32_t str_key;      // a pair key's VARCHAR position (its 32-bit string ids are packed), -1: none

@@ -50,9 +50,10 @@ __device__ __forceinline__ void ctl_publish(Ctl *ctl, Ctl *host) {
 }
 
 struct TableRef {
-    u64 *slots;        // (cap + 2) * stride words
+    u64 *keys;         // cap keys, kstride words apart
+    u64 *states;       // cap + 2 states, stride words apart
     u64 cap;           // power of two
-    int32_t stride;
+    int32_t stride, kstride;
     int32_t gmax_probe;
     Ctl *ctl;
     u64 *spill;        // spill_cap records of (1 + words) words
@@ -189,42 +190,38 @@ __device__ __forceinline__ bool dset_insert_narrow(u64 *set, u64 mask, u64 e, un
     return false;
 }
 
-// Replace each OP_DIST contribution of row r (key pk of kind `kind`, as
-// make_key returns) by 1 if its (group, value) pair is new, else 0.
+// Insert value x of a row with key pk of kind `kind` (as make_key returns)
+// into pair set d; true when the pair is new.
+__device__ __forceinline__ bool dist_insert(const Plan &P, int d, int kind, u64 pk, i64 x) {
+    const u64 slots = P.dmask + 1;
+    if (P.dnarrow)
+        return dset_insert_narrow(P.dsets + slots * d, P.dmask, ((u64)(uint32_t)pk << 32) | (uint32_t)x, P.dmeta, d);
+    u64 *set = P.dsets + 2 * slots * d;
+    u64 g = pk;
+    if (kind == 1) {
+        g = EMPTY_KEY;
+    } else if (kind == 2) {
+        if (P.null_sets) {
+            set = P.null_sets + 2 * slots * d;
+            g = 0;
+        } else {
+            g = DIST_NULL_KEY;
+        }
+    }
+    return dset_insert(set, P.dmask, g, (u64)x, P.dmeta, d);
+}
+
+// Replace each OP_DIST contribution of row r by 1 if its (group, value) pair
+// is new, else 0.
 __device__ __forceinline__ void dist_vals(const Plan &P, u64 r, int kind, u64 pk, u64 *v, u32 *new_pairs) {
 #pragma unroll
     for (int i = 0; i < GB_MAX_OPS; i++) {
         if (i < P.n_ops && P.ops[i].kind == OP_DIST) {
             const Op o = P.ops[i];
             const DevCol &c = P.cols[o.col];
-            u64 x = 0;
-            if (row_valid(c.valid, r) && P.dnarrow) {
-                const u64 e = ((u64)(uint32_t)pk << 32) | (uint32_t)load_int(c, r);
-                if (dset_insert_narrow(P.dsets + (P.dmask + 1) * o.dset, P.dmask, e, P.dmeta, o.dset)) {
-                    x = 1;
-                    atomicAdd(new_pairs, 1u);
-                }
-            } else if (row_valid(c.valid, r)) {
-                const u64 val = (u64)load_int(c, r);
-                const u64 slots = P.dmask + 1;
-                u64 *set = P.dsets + 2 * slots * o.dset;
-                u64 g = pk;
-                if (kind == 1) {
-                    g = EMPTY_KEY;
-                } else if (kind == 2) {
-                    if (P.null_sets) {
-                        set = P.null_sets + 2 * slots * o.dset;
-                        g = 0;
-                    } else {
-                        g = DIST_NULL_KEY;
-                    }
-                }
-                if (dset_insert(set, P.dmask, g, val, P.dmeta, o.dset)) {
-                    x = 1;
-                    atomicAdd(new_pairs, 1u);
-                }
-            }
-            v[i] = x;
+            const bool fresh = row_valid(c.valid, r) && dist_insert(P, o.dset, kind, pk, load_int(c, r));
+            if (fresh) atomicAdd(new_pairs, 1u);
+            v[i] = fresh ? 1 : 0;
         }
     }
 }
@@ -235,8 +232,9 @@ __device__ __forceinline__ void dist_vals(const Plan &P, u64 r, int kind, u64 pk
 __device__ __forceinline__ long long g_slot(const TableRef &T, u64 pk, u64 h, u32 *new_groups) {
     u64 s = h & (T.cap - 1);
     for (int p = 0; p < T.gmax_probe; p++) {
-        u64 *kp = T.slots + s * (u64)T.stride;
-        u64 k = *(volatile u64 *)kp;
+        u64 *kp = T.keys + s * (u64)T.kstride;
+        // a stale free slot (L1) is settled by the compare-and-swap
+        const u64 k = __ldca(kp);
         if (k == pk) return (long long)s;
         if (k == EMPTY_KEY) {
             u64 old = atomicCAS(kp, EMPTY_KEY, pk);
@@ -256,7 +254,7 @@ __device__ __forceinline__ long long g_slot(const TableRef &T, u64 pk, u64 h, u3
 __device__ __forceinline__ long long g_claim(const TableRef &T, u64 pk, u64 home, int p0, u32 *new_groups) {
     for (int p = p0; p < T.gmax_probe; p++) {
         const u64 s = (home + (u64)p) & (T.cap - 1);
-        const u64 old = atomicCAS(T.slots + s * (u64)T.stride, EMPTY_KEY, pk);
+        const u64 old = atomicCAS(T.keys + s * (u64)T.kstride, EMPTY_KEY, pk);
         if (old == EMPTY_KEY) atomicAdd(new_groups, 1u);
         if (old == EMPTY_KEY || old == pk) return (long long)s;
     }
@@ -294,12 +292,12 @@ __device__ __forceinline__ void global_fold(const Plan &P, const TableRef &T, u6
         spill_record(P, T, pk, cnt, v);
         return;
     }
-    apply_state(P, T.slots + (u64)s * (u64)T.stride + 1, cnt, v);
+    apply_state(P, T.states + (u64)s * (u64)T.stride, cnt, v);
 }
 
 // Out-of-band slots (EMPTY_KEY-valued key, NULL key) are folded directly.
 __device__ __forceinline__ void special_fold(const Plan &P, const TableRef &T, int kind, u64 cnt, const u64 *v) {
-    u64 *w = T.slots + (T.cap + (u64)(kind - 1)) * (u64)T.stride + 1;
+    u64 *w = T.states + (T.cap + (u64)(kind - 1)) * (u64)T.stride;
     apply_state(P, w, cnt, v);
 }
 
@@ -554,7 +552,7 @@ __device__ __forceinline__ u64 warp_out_slot(Ctl *ctl, bool occ, unsigned active
 
 // Plan description kept in registers by the fast tile path (up to
 // FAST_MAX_FILTERS predicates on integer or DOUBLE columns; keys SINGLE /
-// PACKED / STRING; any ops but OP_DIST).  kdesc = key_mode | kt0 << 4 | kt1 << 8 | bits_b << 16 |
+// PACKED / STRING; ops over columns).  kdesc = key_mode | kt0 << 4 | kt1 << 8 | bits_b << 16 |
 // bits_a << 24; op[i] = kind | type << 4 | table word << 8 | shared word << 16
 // | wide << 24, wide = a 64-bit shared word (MIN/MAX over BIGINT, the DOUBLE ops).
 struct FastPlan {
@@ -570,6 +568,7 @@ struct FastPlan {
     int32_t eligible;
     int32_t nulls;     // some key, op or filter column has a validity mask
     int32_t flt;       // some op is over DOUBLE
+    int32_t dist;      // some op is OP_DIST
     int32_t sums_f;    // some op is a DOUBLE sum
 };
 

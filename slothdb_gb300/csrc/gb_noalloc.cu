@@ -126,7 +126,7 @@ __global__ void k_merge_noalloc(const __grid_constant__ Plan P, const TableRef T
             continue;
         }
         u64 v[GB_MAX_OPS] = {rec[2]};
-        apply_state(P, T.slots + (u64)s * (u64)T.stride + 1, rec[1], v);
+        apply_state(P, T.states + (u64)s * (u64)T.stride, rec[1], v);
     }
     __syncthreads();
     if (threadIdx.x == 0 && s_new) atomicAdd(&T.ctl->n_groups, s_new);
@@ -207,7 +207,9 @@ extern "C" gb_status gb_hash_aggregate_noalloc(const int64_t *keys, const int64_
     P.stride = kStride;
 
     TableRef T;
-    T.slots = S.table;
+    T.keys = S.table;  // key and state in one slot here
+    T.states = S.table + 1;
+    T.kstride = kStride;
     T.cap = kCap;
     T.stride = kStride;
     T.gmax_probe = 4096;  // at load <= 0.5 a longer probe run does not occur in practice

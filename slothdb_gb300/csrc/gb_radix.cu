@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(P1_WARPS * 32, 1)
                     if (kind == 3) {
                         atomicOr(&T.ctl->err, (u32)ERR_NULL_IN_WIDE_KEY);
                     } else {
-                        u64 *w = T.slots + (T.cap + (u64)(kind - 1)) * (u64)T.stride + 1;
+                        u64 *w = T.states + (T.cap + (u64)(kind - 1)) * (u64)T.stride;
                         fold_atomic<NOPS>(P, w, 1, v);
                     }
                 } else {
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(P1_WARPS * 32, 1)
     const u64 *vcol = (const u64 *)P.cols[R.vcol[0]].data;
     const bool vec = ((((u64)kcol) | ((u64)vcol)) & 15) == 0;
     u64 *hsum = X.hot_part + (u64)blockIdx.x * NH * W + P.ops[0].word;  // this CTA's hot slice, SUM word
-    u64 *oob = T.slots + T.cap * (u64)T.stride + 1;  // state words of the key equal to EMPTY_KEY
+    u64 *oob = T.states + T.cap * (u64)T.stride;  // state words of the key equal to EMPTY_KEY
     const u64 n = A.n_rows;
     const int fop = FILT ? P.filters[0].op : 0;
     const double fdc = FILT ? P.filters[0].dc : 0.0;
