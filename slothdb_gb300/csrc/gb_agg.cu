@@ -215,37 +215,12 @@ __global__ void k_merge_records(const __grid_constant__ Plan P, const u64 *recs,
 // Each CTA takes chunks of `per` * blockDim slots (per <= COMPACT_PER; small
 // tables use fewer slots per thread so that more CTAs share them); one
 // output reservation per chunk.
-#define COMPACT_PER 8
-__global__ void k_compact(const __grid_constant__ Plan P, const u64 *keys, const u64 *states, u64 cap, int stride,
-                          const __grid_constant__ EmitArgs E, Ctl *ctl, int per, Ctl *ctl_host) {
-    const u64 total = cap + 2;
+__global__ void __launch_bounds__(256) k_compact(const __grid_constant__ Plan P, const u64 *keys, const u64 *states,
+                                                 u64 cap, int stride, const __grid_constant__ EmitArgs E, Ctl *ctl,
+                                                 int per, Ctl *ctl_host) {
     const u64 chunk = (u64)per * blockDim.x;
-    for (u64 c0 = blockIdx.x * chunk; c0 < total; c0 += (u64)gridDim.x * chunk) {
-        u32 mine = 0;
-#pragma unroll
-        for (int j = 0; j < COMPACT_PER; j++) {
-            const u64 s = c0 + (u64)j * blockDim.x + threadIdx.x;
-            if (j >= per || s >= total) break;
-            mine += (s < cap) ? (keys[s] != EMPTY_KEY) : (states[s * (u64)stride] != 0);
-        }
-        u64 o = block_out_base(ctl, mine);
-#pragma unroll
-        for (int j = 0; j < COMPACT_PER; j++) {
-            const u64 s = c0 + (u64)j * blockDim.x + threadIdx.x;
-            if (j >= per || s >= total) break;
-            const u64 *sl = states + s * (u64)stride;
-            const u64 k = s < cap ? keys[s] : EMPTY_KEY;
-            const bool occ = (s < cap) ? (k != EMPTY_KEY) : (sl[0] != 0);
-            if (!occ) continue;
-            if (o >= E.out_cap) {
-                atomicOr(&ctl->err, (u32)ERR_OUT_OVERFLOW);
-                continue;
-            }
-            const u64 pk = s <= cap ? k : 0ull;
-            emit_group(P, E, o, pk, s == cap + 1, sl);
-            o++;
-        }
-    }
+    for (u64 c0 = blockIdx.x * chunk; c0 < cap + 2; c0 += (u64)gridDim.x * chunk)
+        compact_chunk(P, E, ctl, keys, states, cap, stride, c0, per);
     __syncthreads();
     if (threadIdx.x == 0) ctl_publish(ctl, ctl_host);
 }

@@ -620,33 +620,8 @@ __global__ void k_batch_compact(const BQuery *qs, const BItem *items, u32 n_item
         copy_words(&sE, &q.E, (int)sizeof(EmitArgs));
         copy_words(&sP, &q.P, (int)sizeof(Plan));
         __syncthreads();
-        const u64 cap = q.T.cap, total = cap + 2;
-        const int stride = q.T.stride;
-        const u64 c0 = (u64)w.idx * (COMPACT_PER * 256);
-        u32 mine = 0;
-#pragma unroll
-        for (int j = 0; j < COMPACT_PER; j++) {
-            const u64 s = c0 + (u64)j * blockDim.x + threadIdx.x;
-            if (s >= total) break;
-            mine += (s < cap) ? (q.T.keys[s] != EMPTY_KEY) : (q.T.states[s * (u64)stride] != 0);
-        }
-        u64 o = block_out_base(q.T.ctl, mine);
-#pragma unroll
-        for (int j = 0; j < COMPACT_PER; j++) {
-            const u64 s = c0 + (u64)j * blockDim.x + threadIdx.x;
-            if (s >= total) break;
-            const u64 *sl = q.T.states + s * (u64)stride;
-            const u64 k = s < cap ? q.T.keys[s] : EMPTY_KEY;
-            const bool occ = (s < cap) ? (k != EMPTY_KEY) : (sl[0] != 0);
-            if (!occ) continue;
-            if (o >= sE.out_cap) {
-                atomicOr(&q.T.ctl->err, (u32)ERR_OUT_OVERFLOW);
-                continue;
-            }
-            const u64 pk = s <= cap ? k : 0ull;
-            emit_group(sP, sE, o, pk, s == cap + 1, sl);
-            o++;
-        }
+        compact_chunk(sP, sE, q.T.ctl, q.T.keys, q.T.states, q.T.cap, q.T.stride, (u64)w.idx * (COMPACT_PER * 256),
+                      COMPACT_PER);
         __syncthreads();
     }
 }
