@@ -80,9 +80,9 @@ __global__ void k_table_init(u64 *table, u64 cap, int stride, const __grid_const
 // last 16).
 struct PackArgs {
     int32_t n;
-    const void *src[2 * (2 + GB_MAX_AGGS) + 1];
-    void *dst[2 * (2 + GB_MAX_AGGS) + 1];
-    u64 vecs[2 * (2 + GB_MAX_AGGS) + 1];
+    const void *src[RESULT_PARTS];
+    void *dst[RESULT_PARTS];
+    u64 vecs[RESULT_PARTS];
 };
 __global__ void k_result_pack(const __grid_constant__ PackArgs A) {
     const u64 me = blockIdx.x * (u64)blockDim.x + threadIdx.x, all = (u64)gridDim.x * blockDim.x;
@@ -679,8 +679,7 @@ struct gb_agg {
     DevBuf types_dev;
     bool topn_applied = false;
     // host result
-    std::vector<HostBuf> host_cols, host_valid;
-    HostBuf host_pack;                      // a small result: all of its columns
+    HostBuf host_pack;                      // all fixed-width columns and validity words
     std::vector<void *> host_col_p, host_valid_p;
     std::vector<const void *> res_ptrs;
     std::vector<const uint64_t *> res_valid;
@@ -2313,8 +2312,6 @@ static void fill_result_view(gb_agg *h, gb_result *out, bool host) {
     out->validity = h->res_valid.data();
 }
 
-#define RESULT_PACK ((size_t)1 << 20)
-
 gb_status gb_agg_result(gb_agg *h, gb_result *out) {
     if (!h || !out) return GB_ERR_INVALID;
     if (!h->finalized) {
@@ -2323,8 +2320,6 @@ gb_status gb_agg_result(gb_agg *h, gb_result *out) {
     }
     if (!h->has_result) {
         size_t nout = h->out_types.size();
-        h->host_cols.resize(nout);
-        h->host_valid.resize(nout);
         h->host_col_p.resize(nout);
         h->host_valid_p.resize(nout);
         u64 n = h->n_rows_out;
@@ -2332,57 +2327,34 @@ gb_status gb_agg_result(gb_agg *h, gb_result *out) {
         auto &cols = h->topn_applied ? h->top_cols : h->out_cols;
         auto &val = h->topn_applied ? h->top_valid : h->out_valid;
         const size_t vbytes = ((size_t)n + 63) / 64 * 8;
-        // fixed-width columns of up to RESULT_PACK bytes: one launch writes them all (gb_agg_result of 64
-        // groups of 5 columns, with its reading in Python: a copy for each column and its validity 45 us, this 35
-        // us); larger ones by the copy engine
         auto width = [&](size_t c) -> size_t {  // a VARCHAR column: its offsets and bytes are copied below
             return h->out_types[c] == GB_T_VARCHAR ? 0 : type_size(h->out_types[c]);
         };
         size_t total = 0;
         for (size_t c = 0; c < nout; c++) total += ((size_t)n * width(c) + 15) / 16 * 16 + (vbytes + 15) / 16 * 16;
-        const bool pack = total <= RESULT_PACK;
-        if (pack && n) {
-            gb_status s = h->host_pack.ensure(total);
-            if (s) return s;
-            PackArgs A;
-            A.n = 0;
-            uint8_t *at = (uint8_t *)h->host_pack.p;
-            u64 most = 0;
-            auto part = [&](const void *src, size_t bytes) -> void * {
-                A.src[A.n] = src;
-                A.dst[A.n] = at;
-                A.vecs[A.n] = (bytes + 15) / 16;
-                most = std::max<u64>(most, A.vecs[A.n]);
-                at += A.vecs[A.n] * 16;
-                return A.dst[A.n++];
-            };
-            for (size_t c = 0; c < nout; c++) {
-                h->host_valid_p[c] = part(val[c].p, vbytes);
-                h->host_col_p[c] = width(c) ? part(cols[c].p, (size_t)n * width(c)) : nullptr;
-            }
-            k_result_pack<<<grid_for(most, 256, sm_count()), 256>>>(A);
-            GB_CUDA(cudaGetLastError());
-        }
+        gb_status s;
+        if ((s = h->host_pack.ensure(total + 16))) return s;
+        gb_part parts[RESULT_PARTS];
+        int np = 0;
+        uint8_t *at = (uint8_t *)h->host_pack.p;
+        auto part = [&](const void *src, size_t bytes) -> void * {
+            parts[np++] = {src, at, bytes};
+            void *p = at;
+            at += (bytes + 15) / 16 * 16;
+            return p;
+        };
         for (size_t c = 0; c < nout; c++) {
-            gb_status s;
-            if (!pack || !n) {
-                if ((s = h->host_valid[c].ensure(vbytes + 8))) return s;
-                h->host_valid_p[c] = h->host_valid[c].p;
-                if (vbytes) GB_CUDA(cudaMemcpyAsync(h->host_valid[c].p, val[c].p, vbytes, cudaMemcpyDeviceToHost, 0));
-            }
-            if (h->out_types[c] == GB_T_VARCHAR) {
-                if ((s = h->host_str_offs.ensure((n + 1) * 8))) return s;
-                GB_CUDA(cudaMemcpy(h->host_str_offs.p, h->out_str_offs.p, (n + 1) * 8, cudaMemcpyDeviceToHost));
-                const int64_t nb = ((const int64_t *)h->host_str_offs.p)[n];
-                if ((s = h->host_str_bytes.ensure((size_t)nb + 8))) return s;
-                if (nb) GB_CUDA(cudaMemcpy(h->host_str_bytes.p, h->out_str_bytes.p, nb, cudaMemcpyDeviceToHost));
-                continue;
-            }
-            if (pack && n) continue;
-            const size_t bytes = (size_t)n * width(c);
-            if ((s = h->host_cols[c].ensure(bytes + 8))) return s;
-            h->host_col_p[c] = h->host_cols[c].p;
-            if (bytes) GB_CUDA(cudaMemcpyAsync(h->host_cols[c].p, cols[c].p, bytes, cudaMemcpyDeviceToHost, 0));
+            h->host_valid_p[c] = part(val[c].p, vbytes);
+            h->host_col_p[c] = part(cols[c].p, (size_t)n * width(c));
+        }
+        if ((s = gb_result_parts(parts, np, 0))) return s;
+        for (size_t c = 0; c < nout; c++) {
+            if (h->out_types[c] != GB_T_VARCHAR) continue;
+            if ((s = h->host_str_offs.ensure((n + 1) * 8))) return s;
+            GB_CUDA(cudaMemcpy(h->host_str_offs.p, h->out_str_offs.p, (n + 1) * 8, cudaMemcpyDeviceToHost));
+            const int64_t nb = ((const int64_t *)h->host_str_offs.p)[n];
+            if ((s = h->host_str_bytes.ensure((size_t)nb + 8))) return s;
+            if (nb) GB_CUDA(cudaMemcpy(h->host_str_bytes.p, h->out_str_bytes.p, nb, cudaMemcpyDeviceToHost));
         }
         GB_CUDA(cudaStreamSynchronize(0));
         h->n_rows_out = n;
@@ -2453,8 +2425,6 @@ void gb_agg_destroy(gb_agg *h) {
     h->topn_ids_b.release();
     h->topn_cnt.release();
     h->types_dev.release();
-    for (auto &b : h->host_cols) b.release();
-    for (auto &b : h->host_valid) b.release();
     for (int i = 0; i < 2; i++) {
         for (auto &b : h->stage[i]) b.release();
         if (h->ev_copied[i]) cudaEventDestroy(h->ev_copied[i]);
@@ -2629,6 +2599,33 @@ gb_status gb_device_sync(void) {
 }
 
 }  // extern "C"
+
+// A copy for each column and its validity took gb_agg_result of 64 groups of 5
+// columns, with its reading in Python, 45 us, one launch 35 us.
+gb_status gb_result_parts(const gb_part *parts, int n, cudaStream_t st) {
+    size_t total = 0;
+    for (int i = 0; i < n; i++) total += parts[i].bytes;
+    if (total > RESULT_PACK || n > RESULT_PARTS) {
+        for (int i = 0; i < n; i++)
+            if (parts[i].bytes)
+                GB_CUDA(cudaMemcpyAsync(parts[i].dst, parts[i].src, parts[i].bytes, cudaMemcpyDeviceToHost, st));
+        return GB_OK;
+    }
+    PackArgs A;
+    A.n = 0;
+    u64 most = 0;
+    for (int i = 0; i < n; i++) {
+        if (!parts[i].bytes) continue;
+        A.src[A.n] = parts[i].src;
+        A.dst[A.n] = parts[i].dst;
+        A.vecs[A.n] = (parts[i].bytes + 15) / 16;
+        most = std::max<u64>(most, A.vecs[A.n++]);
+    }
+    if (!A.n) return GB_OK;
+    k_result_pack<<<grid_for(most, 256, sm_count()), 256, 0, st>>>(A);
+    GB_CUDA(cudaGetLastError());
+    return GB_OK;
+}
 
 // ------------------------------------------------------ Parquet ingest hooks
 gb_status gb_agg_view(gb_agg *h, AggView *v) {

@@ -31,6 +31,17 @@ gb_status gb_agg_ingest_prefiltered_ids(gb_agg *h, const gb_col *cols, uint64_t 
 // until the handle's next encode).
 gb_status gb_agg_encode_strings(gb_agg *h, const uint8_t *bytes, const int64_t *offsets, uint64_t n,
                                 uint64_t total_bytes, void *stream, const int64_t **ids);
+// Parts of a result into page-locked memory, 16 bytes at a time (both sides are
+// aligned and have room for the last 16): one launch for all of them up to
+// RESULT_PACK bytes, else the copy engine.  Not waited for.
+#define RESULT_PACK ((size_t)1 << 20)
+#define RESULT_PARTS (2 * (2 + GB_MAX_AGGS) + 1)
+struct gb_part {
+    const void *src;
+    void *dst;
+    size_t bytes;
+};
+gb_status gb_result_parts(const gb_part *parts, int n, cudaStream_t st);
 // Profiling events around a kernel launched outside gb_agg.cu (no-ops
 // unless the handle's profiling is on).
 struct gb_prof_mark;

@@ -233,3 +233,37 @@ def test_lane_settings(tables):
             capi.check(srv.lib.gb_server_set_lanes(srv.h, 2))  # after the first submit
     finally:
         srv.close()
+
+
+@pytest.mark.parametrize("groups", [0, 1, 63, 64, 65, 32_000, 34_000, 70_000])
+def test_result_copies(groups):
+    """Results of no rows to more than one packed copy takes (1 MB), from the
+    server and from a handle alone, a VARCHAR key's among them."""
+    rng = np.random.default_rng(groups)
+    n = 3 * groups + 1000
+    k = rng.permutation(np.arange(n) % max(groups, 1)).astype(np.int32)
+    v = rng.integers(0 if groups else 10**6, 10**6 if groups else 2 * 10**6, n)
+    text = [b"k%d" % x for x in k]
+    offs = np.zeros(n + 1, np.int64)
+    np.cumsum([len(t) for t in text], out=offs[1:])
+    tabs = [([capi.INTEGER, capi.BIGINT], [k, v]),
+            ([capi.VARCHAR, capi.BIGINT], [(offs, np.frombuffer(b"".join(text), np.uint8).copy()), v])]
+    aggs = [("count_star", -1), ("sum", 1), ("min", 1), ("max", 1)]
+    filters = [(1, "<", 10**6)]
+    srv = capi.Server(budget_bytes=8 << 30, max_batch=8)
+    try:
+        dev = [_dev(c, t) for t, c in tabs]
+        for (types, _), d in zip(tabs, dev):
+            srv.add_table(types, d, n)
+        tickets = [srv.submit(t, 0, n, [0], aggs, filters=filters) for t in (0, 1, 0, 1)]
+        for i, tk in enumerate(tickets):
+            types, cols = tabs[i % 2]
+            want = oracle.run_query(types, [0], aggs, cols, filters=filters)
+            assert srv.wait(tk)
+            out = _out_types(types, [0], aggs)
+            compare(gpu_to_dict(srv.result(tk), 1, out), want)
+            q = dict(r0=0, r1=n, group_cols=[0], aggs=aggs, filters=filters)
+            compare(gpu_to_dict(_alone(types, dev[i % 2], q), 1, out), want)
+            srv.release(tk)
+    finally:
+        srv.close()
