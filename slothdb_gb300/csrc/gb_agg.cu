@@ -1350,7 +1350,7 @@ static gb_status radix_emit(gb_agg *h, cudaStream_t st) {
         TableRef T = table_ref(h);
         RadixRef X = radix_ref(h);
         if (radix_p2_global_words(h->plan, R)) {
-            if ((s = h->r_p2w.ensure((size_t)np * R.sub * (h->plan.words - 1) * 8))) return s;
+            if ((s = h->r_p2w.ensure((size_t)radix_p2_sum_grid(R) * R.sub * (h->plan.words - 1) * 8))) return s;
             X.p2_words = (u64 *)h->r_p2w.p;
         }
         {

@@ -440,10 +440,8 @@ __device__ __forceinline__ i64 sext(u64 x, int bits) {
 }
 
 
-// Write one group's result row `o` (key columns + finalised aggregates,
-// agg_emit_helpers.cpp:26-98 rules).  `w` = the group's state words.
-__device__ __forceinline__ void emit_group(const Plan &P, const EmitArgs &E, u64 o, u64 pk, bool null_key,
-                                           const u64 *w) {
+// The key columns of result row `o`.
+__device__ __forceinline__ void emit_key(const Plan &P, const EmitArgs &E, u64 o, u64 pk, bool null_key) {
     if (P.key_mode == KEY_SINGLE || P.key_mode == KEY_STRING) {
         store_int(E.out[0], P.key_type[0], o, (i64)pk);
         if (null_key) clear_valid(E.valid[0], o);
@@ -460,6 +458,13 @@ __device__ __forceinline__ void emit_group(const Plan &P, const EmitArgs &E, u64
         store_int(E.out[0], P.str_key == 0 ? GB_T_BIGINT : P.key_type[0], o, (i64)(int32_t)(uint32_t)(pk >> 32));
         store_int(E.out[1], P.str_key == 1 ? GB_T_BIGINT : P.key_type[1], o, (i64)(int32_t)(uint32_t)pk);
     }
+}
+
+// Write one group's result row `o` (key columns + finalised aggregates,
+// agg_emit_helpers.cpp:26-98 rules).  `w` = the group's state words.
+__device__ __forceinline__ void emit_group(const Plan &P, const EmitArgs &E, u64 o, u64 pk, bool null_key,
+                                           const u64 *w) {
+    emit_key(P, E, o, pk, null_key);
     for (int a = 0; a < E.n_aggs; a++) {
         const EmitAgg &g = E.aggs[a];
         void *dst = E.out[E.n_keys + a];

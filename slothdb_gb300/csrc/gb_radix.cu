@@ -58,14 +58,43 @@ __device__ __forceinline__ u32 hot_bucket(u64 h, int HB) { return (u32)(h >> 32)
 __device__ __forceinline__ u32 agg_slot(u64 h, int SP) { return (u32)(h >> 20) & (u32)(SP - 1); }
 
 // ------------------------------------------------------------- sampling
-__global__ void k_sample_count(const __grid_constant__ Plan P, u64 n, u64 step, u64 m, u64 *skeys, u32 *scnt,
-                               u64 scap) {
-    for (u64 i = blockIdx.x * (u64)blockDim.x + threadIdx.x; i < m; i += (u64)gridDim.x * blockDim.x) {
+// A block counts its rows in shared memory first: one row in nine of a Zipf
+// column is the same key, whose count in HBM the rows took in turn (100M rows,
+// the four launches of a sample: 109 -> 89 us).
+#define SAMPLE_ROWS 1536  // rows of a block
+#define SAMPLE_SLOTS 2048
+__global__ void __launch_bounds__(512) k_sample_count(const __grid_constant__ Plan P, u64 n, u64 step, u64 m,
+                                                      u64 *skeys, u32 *scnt, u64 scap) {
+    __shared__ u64 keys[SAMPLE_SLOTS];
+    __shared__ u32 cnt[SAMPLE_SLOTS];
+    for (int i = threadIdx.x; i < SAMPLE_SLOTS; i += blockDim.x) {
+        keys[i] = EMPTY_KEY;
+        cnt[i] = 0;
+    }
+    __syncthreads();
+    const u64 i1 = min(m, (u64)(blockIdx.x + 1) * SAMPLE_ROWS);
+    for (u64 i = (u64)blockIdx.x * SAMPLE_ROWS + threadIdx.x; i < i1; i += blockDim.x) {
         const u64 r = i * step;
         if (r >= n) continue;
         if (P.n_filters && !pass_filters(P, r)) continue;
         u64 pk;
         if (make_key(P, r, pk) != 0) continue;
+        u32 s = (u32)mix64(pk) & (SAMPLE_SLOTS - 1);
+        for (int p = 0; p < SAMPLE_SLOTS; p++) {
+            u64 k = *(volatile u64 *)&keys[s];
+            if (k == EMPTY_KEY) {
+                const u64 old = atomicCAS(&keys[s], EMPTY_KEY, pk);
+                k = old == EMPTY_KEY ? pk : old;
+            }
+            if (k == pk) break;
+            s = (s + 1) & (SAMPLE_SLOTS - 1);
+        }
+        atomicAdd(&cnt[s], 1u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < SAMPLE_SLOTS; i += blockDim.x) {
+        const u64 pk = keys[i];
+        if (pk == EMPTY_KEY) continue;
         u64 s = mix64(pk) & (scap - 1);
         for (u64 p = 0; p < scap; p++) {
             u64 k = *(volatile u64 *)&skeys[s];
@@ -74,7 +103,7 @@ __global__ void k_sample_count(const __grid_constant__ Plan P, u64 n, u64 step, 
                 if (old == EMPTY_KEY || old == pk) k = pk;
             }
             if (k == pk) {
-                atomicAdd(&scnt[s], 1u);
+                atomicAdd(&scnt[s], cnt[i]);
                 break;
             }
             s = (s + 1) & (scap - 1);
@@ -254,6 +283,12 @@ __device__ __forceinline__ void tuple_contrib(const Plan &P, const RadixPlan &R,
         default: v[i] = x; break;
         }
     }
+}
+
+// A DOUBLE sum in L2 that nothing waits for (k_part_agg_sum's atomicAdds went
+// out as the returning form).
+__device__ __forceinline__ void red_f64(u64 *w, double x) {
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(w)), "d"(x) : "memory");
 }
 
 // Plain (non-atomic) fold of a combined partial into state words owned by
@@ -771,6 +806,17 @@ __global__ void k_fill_u64(u64 *dst, u64 n, u64 value) {
 }
 
 // ------------------------------------------------------------- P2 aggregate
+// The first output row of each warp's slots (warp w owns slots [w, w + 1) *
+// SP / warps): one output reservation per CTA.  Warps then write
+// their used slots as consecutive rows (a run of rows per thread instead
+// scattered every store over 32 rows).
+__device__ __forceinline__ u64 warp_out_base(Ctl *ctl, const u64 *keys, int SP) {
+    const int per = SP / (int)(blockDim.x / 32), s0 = (threadIdx.x >> 5) * per + (threadIdx.x & 31);
+    u32 mine = 0;
+    for (int i = 0; i < per; i += 32) mine += keys[s0 + i] != EMPTY_KEY;
+    return __shfl_sync(FULL, block_out_base(ctl, mine), 0);
+}
+
 // One CTA per partition: a shared open-addressing table (u64 keys, u32
 // counts, W-1 state words).  Warps pre-combine duplicate keys, then fold with
 // native u32 count atomics and (rarely contended) word atomics; no barriers
@@ -899,21 +945,21 @@ __global__ void __launch_bounds__(RADIX_BLOCK, 1)
         if (!done) global_fold_n<NOPS>(P, T, pk, cnt, v, &s_new);
     }
     __syncthreads();
-    // emit: one output reservation per CTA
-    u32 mine = 0;
-    for (int s = threadIdx.x; s < SP; s += blockDim.x) mine += keys[s] != EMPTY_KEY;
-    u64 o = block_out_base(T.ctl, mine);
-    for (int s = threadIdx.x; s < SP; s += blockDim.x) {
-        if (keys[s] == EMPTY_KEY) continue;
-        if (o >= E.out_cap) {
-            atomicOr(&T.ctl->err, (u32)ERR_OUT_OVERFLOW);
-            continue;
+    u64 o = warp_out_base(T.ctl, keys, SP);
+    const int per = SP / (RADIX_BLOCK / 32);
+    for (int s0 = (threadIdx.x >> 5) * per; s0 < ((int)(threadIdx.x >> 5) + 1) * per; s0 += 32) {
+        const int s = s0 + lane;
+        const u64 k = keys[s];
+        const unsigned used = __ballot_sync(FULL, k != EMPTY_KEY);
+        if (k != EMPTY_KEY) {
+            const u64 row = o + __popc(used & ((1u << lane) - 1u));
+            u64 w[GB_MAX_WORDS];
+            w[0] = cn[s];
+            for (int q = 0; q < WM; q++) w[1 + q] = wd[(size_t)s * WM + q];
+            if (row < E.out_cap) emit_group(P, E, row, k, false, w);
+            else atomicOr(&T.ctl->err, (u32)ERR_OUT_OVERFLOW);
         }
-        u64 w[GB_MAX_WORDS];
-        w[0] = cn[s];
-        for (int q = 0; q < WM; q++) w[1 + q] = wd[(size_t)s * WM + q];
-        emit_group(P, E, o, keys[s], false, w);
-        o++;
+        o += __popc(used);
     }
     __syncthreads();
     if (threadIdx.x == 0 && s_new) atomicAdd(&T.ctl->n_groups, s_new);
@@ -921,89 +967,160 @@ __global__ void __launch_bounds__(RADIX_BLOCK, 1)
 
 // P2 for plans whose ops are all DOUBLE SUMs of the one value column (the
 // COUNT / SUM / AVG(DOUBLE) shape): shared memory holds only keys and u32
-// counts; the sum words of this partition live in its slice of p2_words and
-// fold as fire-and-forget L2 reductions.  The CTA zeroes its slice first:
-// full-line stores allocate the lines in L2 without a DRAM read, so the
-// reductions that follow hit L2 (a slice left zero between runs instead made
-// every first reduction of a line miss).  One 128-bit load per tuple, no
-// per-op switch; the slot comes from bits 20.. of the P1 hash (the partition
-// took its top bits).
+// counts; the sum words live in the CTA's slice of p2_words and fold as
+// fire-and-forget L2 reductions.  The slot comes from bits 20.. of the P1 hash
+// (the partition took its top bits).  A CTA takes partitions blockIdx,
+// blockIdx + grid, ..., so its slice stays in L2; the emit leaves the slots
+// that it reads empty for the next partition, whose tuples head for L2
+// meanwhile.  Two CTAs share an SM where tables of half the size hold the
+// estimate: one probes while the other divides and writes.  28.5M tuples of
+// 6.2M groups, tables of 8192 slots: 739 -> 510 us (717 with the words of one
+// round of slots read at a time: the emit waited for L2).
+template <int NOPS>
+__device__ __noinline__ void p2_sum_overflow(const Plan &P, const TableRef &T, u64 pk, u64 x, u32 *new_groups) {
+    u64 v[NOPS];
+#pragma unroll
+    for (int o = 0; o < NOPS; o++) v[o] = x;
+    global_fold_n<NOPS>(P, T, pk, 1, v, new_groups);
+}
+
+// The slot of pk past home slot s, which holds another key (SP: none within `probe`).
+__device__ __forceinline__ u32 p2_walk(u64 *keys, int SP, int probe, u32 s, u64 pk) {
+    volatile u64 *vk = keys;
+#pragma unroll 1
+    for (int q = 1; q < probe; q++) {
+        s = (s + 1) & (u32)(SP - 1);
+        u64 k = vk[s];
+        if (k == EMPTY_KEY) {
+            const u64 old = atomicCAS(&keys[s], EMPTY_KEY, pk);
+            k = (old == EMPTY_KEY) ? pk : old;
+        }
+        if (k == pk) return s;
+    }
+    return (u32)SP;
+}
+
 template <int NOPS>
 __global__ void __launch_bounds__(RADIX_BLOCK, 1)
     k_part_agg_sum(const __grid_constant__ Plan P, const __grid_constant__ RadixPlan R, const RadixRef X,
-                   const TableRef T, const __grid_constant__ EmitArgs E, int SP) {
+                   const __grid_constant__ TableRef T, const __grid_constant__ EmitArgs E, int SP) {
     extern __shared__ u64 rsm[];
-    const int WM = P.words - 1;
+    const u32 np = 1u << R.pbits;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     u64 *keys = rsm;               // [SP]
     u32 *cn = (u32 *)(keys + SP);  // [SP]
-    u64 *wd = X.p2_words + (size_t)blockIdx.x * SP * WM;  // [SP][WM]
+    u64 *wd = X.p2_words + (size_t)blockIdx.x * SP * NOPS;  // [SP][NOPS]
     __shared__ u32 s_new;
     for (int i = threadIdx.x; i < SP; i += blockDim.x) {
         keys[i] = EMPTY_KEY;
         cn[i] = 0;
     }
-    for (int i = threadIdx.x; i < SP * WM; i += blockDim.x) wd[i] = 0ull;  // DOUBLE SUM identity
+    for (int i = threadIdx.x; i < SP * NOPS; i += blockDim.x) wd[i] = 0ull;  // DOUBLE SUM identity
     if (threadIdx.x == 0) s_new = 0;
-    const u32 p = blockIdx.x;
-    const u64 n = min((u64)X.cursor[(u64)p * CURSOR_PAD], (u64)X.part_cap[p]);
-    const ulonglong2 *base = (const ulonglong2 *)(X.part + X.part_off[p] * 2);
-    if (threadIdx.x < 32) {
-        const u64 bytes = n * 16, piece = 32768;
-        for (u64 o = (u64)threadIdx.x * piece; o < bytes; o += 32 * piece)
-            l2_prefetch((const char *)base + o, min(piece, bytes - o));
-    }
-    int wo[NOPS];
-#pragma unroll
-    for (int o = 0; o < NOPS; o++) wo[o] = P.ops[o].word - 1;
-    __syncthreads();
     volatile u64 *vk = keys;
-    for (u64 i = threadIdx.x; i < n; i += blockDim.x) {
-        const ulonglong2 t = __ldcs(base + i);
-        const u64 pk = t.x;
-        if (pk == EMPTY_KEY) continue;  // a padding hole of the write-combining P1
-        u32 s = agg_slot(p1_hash(pk), SP);
-        bool done = false;
-        for (int q = 0; q < R.agg_probe; q++) {
-            u64 k = vk[s];
-            if (k == EMPTY_KEY) {
-                const u64 old = atomicCAS(&keys[s], EMPTY_KEY, pk);
-                k = (old == EMPTY_KEY) ? pk : old;
-            }
-            if (k == pk) {
-                atomicAdd(&cn[s], 1u);
-#pragma unroll
-                for (int o = 0; o < NOPS; o++)
-                    atomicAdd((double *)(wd + (size_t)s * WM + wo[o]), __longlong_as_double((i64)t.y));
-                done = true;
-                break;
-            }
-            s = (s + 1) & (u32)(SP - 1);
-        }
-        if (!done) {
-            u64 v[NOPS];
-#pragma unroll
-            for (int o = 0; o < NOPS; o++) v[o] = t.y;
-            global_fold_n<NOPS>(P, T, pk, 1, v, &s_new);
-        }
-    }
-    __threadfence();  // the reductions reach L2 before the emit reads them
+    auto prefetch = [&](u32 p) {  // a warp: 32 KB pieces, one per lane
+        const u64 bytes = min((u64)X.cursor[(u64)p * CURSOR_PAD], (u64)X.part_cap[p]) * 16, piece = 32768;
+        const char *base = (const char *)(X.part + X.part_off[p] * 2);
+        for (u64 o = (u64)lane * piece; o < bytes; o += 32 * piece) l2_prefetch(base + o, min(piece, bytes - o));
+    };
+    if (warp == 0) prefetch(blockIdx.x);
     __syncthreads();
-    u32 mine = 0;
-    for (int s = threadIdx.x; s < SP; s += blockDim.x) mine += keys[s] != EMPTY_KEY;
-    u64 o = block_out_base(T.ctl, mine);
-    for (int s = threadIdx.x; s < SP; s += blockDim.x) {
-        if (keys[s] == EMPTY_KEY) continue;
-        if (o >= E.out_cap) {
-            atomicOr(&T.ctl->err, (u32)ERR_OUT_OVERFLOW);
-            continue;
+    for (u32 p = blockIdx.x; p < np; p += gridDim.x) {
+        const u64 n = min((u64)X.cursor[(u64)p * CURSOR_PAD], (u64)X.part_cap[p]);
+        const ulonglong2 *base = (const ulonglong2 *)(X.part + X.part_off[p] * 2);
+        if (warp == 0 && p + gridDim.x < np) prefetch(p + gridDim.x);
+        const u64 step = (u64)P2_ROWS * blockDim.x;
+        ulonglong2 t[P2_ROWS], next[P2_ROWS];
+        auto load = [&](ulonglong2 *to, u64 at) {
+#pragma unroll
+            for (int j = 0; j < P2_ROWS; j++) {
+                const u64 i = at + (u64)j * blockDim.x + threadIdx.x;
+                to[j] = i < n ? __ldcs(base + i) : make_ulonglong2(EMPTY_KEY, 0ull);
+            }
+        };
+        load(next, 0);
+        for (u64 b0 = 0; b0 < n; b0 += step) {
+            u32 at[P2_ROWS];  // slot, SP: none found
+            u64 k[P2_ROWS];
+#pragma unroll
+            for (int j = 0; j < P2_ROWS; j++) t[j] = next[j];
+            load(next, b0 + step);
+            // the home slots of all tuples in flight, then the few that go on
+#pragma unroll
+            for (int j = 0; j < P2_ROWS; j++) {
+                at[j] = agg_slot(p1_hash(t[j].x), SP);
+                k[j] = vk[at[j]];
+            }
+#pragma unroll
+            for (int j = 0; j < P2_ROWS; j++) {
+                if (k[j] != EMPTY_KEY || t[j].x == EMPTY_KEY) continue;
+                const u64 old = atomicCAS(&keys[at[j]], EMPTY_KEY, t[j].x);
+                k[j] = (old == EMPTY_KEY) ? t[j].x : old;
+            }
+#pragma unroll
+            for (int j = 0; j < P2_ROWS; j++)
+                if (k[j] != t[j].x && t[j].x != EMPTY_KEY) at[j] = p2_walk(keys, SP, R.agg_probe, at[j], t[j].x);
+            __syncwarp();  // the lanes' atomics go out together, however long each probed
+#pragma unroll
+            for (int j = 0; j < P2_ROWS; j++) {
+                if (t[j].x == EMPTY_KEY) continue;  // no tuple, or a padding hole of the write-combining P1
+                if (at[j] < (u32)SP) {
+                    atomicAdd(&cn[at[j]], 1u);
+#pragma unroll
+                    for (int o = 0; o < NOPS; o++)
+                        red_f64(wd + (size_t)at[j] * NOPS + o, __longlong_as_double((i64)t[j].y));
+                } else {
+                    p2_sum_overflow<NOPS>(P, T, t[j].x, t[j].y, &s_new);
+                }
+            }
         }
-        u64 w[GB_MAX_WORDS];
-        w[0] = cn[s];
-        for (int q = 0; q < WM; q++) w[1 + q] = __ldcg(wd + (size_t)s * WM + q);
-        emit_group(P, E, o, keys[s], false, w);
-        o++;
+        __threadfence();  // the reductions reach L2 before the emit reads them
+        __syncthreads();
+        // every op is a SUM of the value column in words 1.., and no value is
+        // NULL: a COUNT is the count, a SUM a word, an AVG their quotient
+        u64 o = warp_out_base(T.ctl, keys, SP);
+        const int per = SP / (int)(blockDim.x / 32);
+        for (int s0 = warp * per; s0 < (warp + 1) * per; s0 += 32 * P2_EMIT) {
+            // a few rounds' words in flight (one at a time the reads of L2 took half of the kernel)
+            u64 k[P2_EMIT], w[P2_EMIT][NOPS];
+#pragma unroll
+            for (int e = 0; e < P2_EMIT; e++) {
+                const int s = s0 + 32 * e + lane;
+                k[e] = keys[s];
+#pragma unroll
+                for (int q = 0; q < NOPS; q++) w[e][q] = k[e] != EMPTY_KEY ? __ldcg(wd + (size_t)s * NOPS + q) : 0ull;
+            }
+#pragma unroll
+            for (int e = 0; e < P2_EMIT; e++) {
+                const int s = s0 + 32 * e + lane;
+                const unsigned used = __ballot_sync(FULL, k[e] != EMPTY_KEY);
+                if (k[e] != EMPTY_KEY) {
+                    const u64 row = o + __popc(used & ((1u << lane) - 1u));
+                    const u32 cnt = cn[s];
+                    keys[s] = EMPTY_KEY;
+                    cn[s] = 0;
+#pragma unroll
+                    for (int q = 0; q < NOPS; q++) wd[(size_t)s * NOPS + q] = 0ull;
+                    if (row < E.out_cap) {
+                        emit_key(P, E, row, k[e], false);
+                        for (int a = 0; a < E.n_aggs; a++) {
+                            const EmitAgg &g = E.aggs[a];
+                            const u64 x = NOPS == 1 || g.val_word == 1 ? w[e][0] : w[e][NOPS - 1];
+                            u64 *dst = (u64 *)E.out[E.n_keys + a] + row;
+                            if (g.kind == GB_AGG_SUM) *dst = x;
+                            else if (g.kind == GB_AGG_AVG)
+                                *(double *)dst = __longlong_as_double((i64)x) / (double)cnt;
+                            else *dst = cnt;
+                        }
+                    } else {
+                        atomicOr(&T.ctl->err, (u32)ERR_OUT_OVERFLOW);
+                    }
+                }
+                o += __popc(used);
+            }
+        }
+        __syncthreads();  // the slots are empty again
     }
-    __syncthreads();
     if (threadIdx.x == 0 && s_new) atomicAdd(&T.ctl->n_groups, s_new);
 }
 
@@ -1079,6 +1196,9 @@ bool radix_p2_global_words(const Plan &P, const RadixPlan &R) {
     return true;
 }
 
+// CTAs of k_part_agg_sum, each with its own slice of words.
+int radix_p2_sum_grid(const RadixPlan &R) { return std::min(1 << R.pbits, sm_count() * (P2_SUB_MAX / R.sub)); }
+
 // Rows of one claim of the P1 kernel that runs (a CTA tile of the generic
 // kernel, a warp claim of the specialised one) and the rows that can still be
 // in flight when the kernel is told to stop (every claim is finished).
@@ -1107,6 +1227,7 @@ static int p1_spec(const Plan &P, const RadixPlan &R, u64 nullable_mask) {
 
 int radix_spec_of(const Plan &P, const RadixPlan &R, u64 nullable_mask) { return p1_spec(P, R, nullable_mask); }
 
+static_assert(P2_SUB_MAX * 12 <= 224 * 1024 && 2 * (P2_SUB_MAX / 2 * 12 + 1024) <= 224 * 1024, "tables of k_part_agg_sum");
 static const size_t kSmemBudget = 224 * 1024;  // <= the 227 KiB opt-in minus static shared memory
 
 gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullable_mask) {
@@ -1135,11 +1256,12 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
     // 12 bytes a slot, when the state words fold in L2)
     int sp = 8192;
     R.sub = sp;
-    if (radix_p2_global_words(P, R) && (size_t)16384 * 12 <= kSmemBudget) {
-        sp = 16384;
+    const u64 max_np = 4096;
+    if (radix_p2_global_words(P, R) && est_groups > max_np * (sp * 7 / 10)) {
+        sp = P2_SUB_MAX;
         R.sub = sp;
     }
-    while (sp > 512 && !radix_p2_global_words(P, R) && radix_p2_smem(P, R) > kSmemBudget) {
+    while (sp > 1024 && !radix_p2_global_words(P, R) && radix_p2_smem(P, R) > kSmemBudget) {
         sp /= 2;
         R.sub = sp;
     }
@@ -1149,7 +1271,7 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
     // partitions so that a partition's groups fill its table to <= ~0.7
     const u64 per_part = (u64)sp * 7 / 10;
     u64 np = pow2_at_least(std::max<u64>((est_groups + per_part - 1) / per_part, 64));
-    np = std::min<u64>(np, 4096);
+    np = std::min<u64>(np, max_np);
     int pb = 0;
     while ((1ull << pb) < np) pb++;
     R.pbits = pb;
@@ -1202,7 +1324,7 @@ gb_status radix_launch_sample(const Plan &P, const RadixPlan &R, u64 n, u64 *ske
     const u64 m = std::min<u64>(n, scap / 2);
     const u64 step = std::max<u64>(1, n / std::max<u64>(m, 1));
     const int sms = sm_count();
-    k_sample_count<<<grid_of(m, 256, sms * 4), 256, 0, st>>>(P, n, step, m, skeys, scnt, scap);
+    k_sample_count<<<(int)((m + SAMPLE_ROWS - 1) / SAMPLE_ROWS), 512, 0, st>>>(P, n, step, m, skeys, scnt, scap);
     k_sample_hist<<<grid_of(scap, 256, sms * 2), 256, 0, st>>>(skeys, scnt, scap, hist);
     k_hot_collect<<<grid_of(scap, 256, sms * 2), 256, 0, st>>>(skeys, scnt, scap, hist, hstate, R.nh, cand_key,
                                                               cand_cnt);
@@ -1307,13 +1429,15 @@ gb_status radix_launch_p2(const Plan &P, const RadixPlan &R, const RadixRef &X, 
     gb_status s = radix_set_attributes();
     if (s) return s;
     size_t smem = radix_p2_smem(P, R);
-    const int np = 1 << R.pbits;
+    int grid = 1 << R.pbits, block = RADIX_BLOCK;
     P2Fn f = g_p2[R.V * (RADIX_MAX_OPS + 1) + P.n_ops];
     if (X.p2_words && radix_p2_global_words(P, R)) {
         f = g_p2_gw[P.n_ops];
         smem = (size_t)R.sub * 12;
+        grid = radix_p2_sum_grid(R);
+        block = RADIX_BLOCK / (P2_SUB_MAX / R.sub);
     }
-    f<<<np, RADIX_BLOCK, smem, st>>>(P, R, X, T, E, R.sub);
+    f<<<grid, block, smem, st>>>(P, R, X, T, E, R.sub);
     GB_CUDA(cudaGetLastError());
     return GB_OK;
 }

@@ -10,6 +10,9 @@
 #define P1_WARPS 32   // P1 block = 1024 threads (64 registers each: 32 warps per SM)
 #define REG_HOT 4     // hottest keys accumulated in per-lane registers
 #define RADIX_BLOCK 1024
+#define P2_SUB_MAX 16384  // slots of k_part_agg_sum's tables: one CTA per SM, or two of half the slots and threads
+#define P2_EMIT 4     // rounds of 32 slots whose words are read together (k_part_agg_sum)
+#define P2_ROWS 2     // tuples of a thread in flight (k_part_agg_sum)
 #define CURSOR_PAD 32    // partition cursors 128 bytes apart (spread over L2 slices)
 #define HIST_BINS 1024   // sample-count histogram bins
 
@@ -44,7 +47,7 @@ struct RadixRef {
     const uint16_t *hot_idx;  // hot rank of each bucket slot
     const u64 *hot_list;      // nh keys by hot index
     u64 *hot_part;            // [grid][nh][words] per-CTA hot partials
-    u64 *p2_words;            // [np][sub][words - 1] P2 state words when they fold in L2 (or null)
+    u64 *p2_words;            // [CTA][sub][words - 1] P2 state words when they fold in L2 (or null)
 };
 
 struct RadixTile {
@@ -61,6 +64,7 @@ gb_status radix_set_bits(const Plan &P, RadixPlan &R, int bits);
 int radix_spec_of(const Plan &P, const RadixPlan &R, u64 nullable_mask);
 size_t radix_p2_smem(const Plan &P, const RadixPlan &R);
 bool radix_p2_global_words(const Plan &P, const RadixPlan &R);
+int radix_p2_sum_grid(const RadixPlan &R);
 u32 radix_tile_rows(const RadixPlan &R);
 u64 radix_inflight_rows(const RadixPlan &R, int grid);
 size_t radix_p1d_smem(const RadixPlan &R);
