@@ -269,6 +269,36 @@ __device__ __forceinline__ void topn_code(const TopnArgs &A, u64 i, u64 &p, u64 
     }
 }
 
+// The primary codes of N rows (~0u: none, code ~0), their loads in flight
+// together: the type is switched on outside.
+template <int N>
+__device__ __forceinline__ void topn_primary(const TopnArgs &A, const u32 *row, u64 *p) {
+    u64 word[N];
+    i64 x[N];
+#pragma unroll
+    for (int j = 0; j < N; j++) word[j] = A.order_valid && row[j] != ~0u ? A.order_valid[row[j] >> 6] : ~0ull;
+    switch (A.order_type) {
+    case GB_T_SMALLINT:
+#pragma unroll
+        for (int j = 0; j < N; j++) x[j] = row[j] != ~0u ? (i64)((const int16_t *)A.order_col)[row[j]] : 0;
+        break;
+    case GB_T_INTEGER:
+#pragma unroll
+        for (int j = 0; j < N; j++) x[j] = row[j] != ~0u ? (i64)((const int32_t *)A.order_col)[row[j]] : 0;
+        break;
+    default:
+#pragma unroll
+        for (int j = 0; j < N; j++) x[j] = row[j] != ~0u ? ((const i64 *)A.order_col)[row[j]] : 0;
+        break;
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        u64 prim = ord_u64(A.order_type == GB_T_DOUBLE ? enc_f64(__longlong_as_double(x[j])) : x[j]);
+        if (!((word[j] >> (row[j] & 63)) & 1ull)) prim = 0;  // NULL, as in topn_code
+        p[j] = row[j] == ~0u ? ~0ull : (A.ascending ? prim : ~prim);
+    }
+}
+
 __device__ __forceinline__ bool code_less(u64 ap, u64 as, u64 bp, u64 bs) {
     return ap < bp || (ap == bp && as < bs);
 }
@@ -440,10 +470,12 @@ __global__ void __launch_bounds__(512) k_topn(const __grid_constant__ TopnArgs A
 }
 
 // TopN for K <= 32: each warp keeps its best K rows in registers, sorted
-// (lane i holds the i-th best; lanes >= K hold nothing); a row better than
-// the warp's K-th enters by one shuffle insertion.  Warp 0 then merges the
-// block's warp lists the same way.  Items: result rows (ids == nullptr) or a
-// candidate list of row ids (~0u = none).  Output: the block's best K ids in
+// (lane i holds the i-th best; lanes >= K hold nothing).  Rows no better than
+// the K-th of any warp of the block are passed over; of 32 rows, a few enter
+// one by one, more are sorted and merged with the list.  The block's lists are
+// merged pairwise.  Items: result rows (ids == nullptr) or the sorted
+// candidate lists of `lists` blocks, K row ids each (~0u = none), their heads
+// first.  The best 10 of 6.2M rows: 92 -> 58 us.  Output: the block's best K ids in
 // out_ids[blockIdx.x * K + i] (~0u past out_n[blockIdx.x]).
 struct TopItem {
     u64 p, s;
@@ -471,71 +503,132 @@ __device__ __forceinline__ void warp_list_insert(TopItem &mine, int K, u64 p, u6
     }
 }
 
+// A total order: equal codes by row, no row (~0u) last.
+__device__ __forceinline__ bool item_less(const TopItem &a, const TopItem &b) {
+    return code_less(a.p, a.s, b.p, b.s) || (a.p == b.p && a.s == b.s && a.id < b.id);
+}
+
+// Lane i takes the smaller (low) or larger of its item and lane i ^ mask's.
+__device__ __forceinline__ void item_exchange(TopItem &a, int mask, bool low) {
+    TopItem b;
+    b.p = __shfl_xor_sync(FULL, a.p, mask);
+    b.s = __shfl_xor_sync(FULL, a.s, mask);
+    b.id = __shfl_xor_sync(FULL, a.id, mask);
+    if (low ? item_less(b, a) : item_less(a, b)) a = b;
+}
+
+__device__ __forceinline__ void warp_sort(TopItem &a) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll 1
+        for (int o = size >> 1; o; o >>= 1) item_exchange(a, o, ((lane & o) == 0) == ((lane & size) == 0));
+}
+
+// mine := the best K of two sorted lists.
+__device__ __forceinline__ void warp_list_merge(TopItem &mine, TopItem other, int K) {
+    const int lane = threadIdx.x & 31;
+    TopItem b;
+    b.p = __shfl_sync(FULL, other.p, 31 - lane);
+    b.s = __shfl_sync(FULL, other.s, 31 - lane);
+    b.id = __shfl_sync(FULL, other.id, 31 - lane);
+    if (item_less(b, mine)) mine = b;  // the 32 best, a bitonic sequence
+#pragma unroll 1
+    for (int o = 16; o; o >>= 1) item_exchange(mine, o, (lane & o) == 0);
+    if (lane >= K) mine = TopItem{~0ull, ~0ull, ~0u};
+}
+
 __global__ void __launch_bounds__(512) k_topn_small(const __grid_constant__ TopnArgs A, const u32 *ids, u64 n,
-                                                    u32 *out_ids, u32 *out_n) {
+                                                    int lists, u32 *out_ids, u32 *out_n) {
     __shared__ TopItem s_list[16][32];
+    __shared__ unsigned long long s_bound;  // the best of the warps' K-th codes
+    __shared__ u64 s_best[16];              // each warp's best code so far
     const int K = A.K;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    if (threadIdx.x == 0) s_bound = ~0ull;
+    if (threadIdx.x < 16) s_best[threadIdx.x] = ~0ull;
+    __syncthreads();
     TopItem mine{~0ull, ~0ull, ~0u};
     const u64 per = (n + gridDim.x - 1) / gridDim.x;
     const u64 lo = blockIdx.x * per, hi = min(n, lo + per);
     constexpr int TR = 4;  // rows per lane per step: their loads are issued together
     u64 tp = ~0ull, ts = ~0ull;  // the warp's K-th best
     bool full = false;           // K rows held: only better rows enter
-    for (u64 base = lo + (u64)warp * 32 * TR; base < hi; base += (u64)nwarps * 32 * TR) {
-        u64 cp[TR], cs[TR];
-        u32 row[TR];
+    u64 mybest = ~0ull;
+    for (u64 base0 = lo; base0 < hi; base0 += (u64)nwarps * 32 * TR) {
+        const u64 base = base0 + (u64)warp * 32 * TR;
+        TopItem c[TR];
 #pragma unroll
         for (int j = 0; j < TR; j++) {
             const u64 it = base + (u64)j * 32 + lane;
-            cp[j] = cs[j] = ~0ull;
-            row[j] = ~0u;
+            c[j] = TopItem{~0ull, ~0ull, ~0u};
             if (it < hi) {
-                row[j] = ids ? ids[it] : (u32)it;
-                if (row[j] != ~0u) topn_code(A, row[j], cp[j], cs[j]);
+                c[j].id = ids ? ids[it % lists * K + it / lists] : (u32)it;
             }
+        }
+        u32 row[TR];
+        u64 prim[TR];
+#pragma unroll
+        for (int j = 0; j < TR; j++) row[j] = c[j].id;
+        topn_primary<TR>(A, row, prim);
+        u64 pass = ~0ull;
+        if (K <= nwarps) {
+            // no row past the K-th of the warps' best rows is among the best K
+            u64 b = prim[0];
+#pragma unroll
+            for (int j = 1; j < TR; j++) b = min(b, prim[j]);
+            for (int o = 16; o; o >>= 1) b = min(b, __shfl_xor_sync(FULL, b, o));
+            if (b < mybest) {
+                mybest = b;
+                if (lane == 0) *(volatile u64 *)&s_best[warp] = b;
+            }
+            if (base0 == lo) __syncthreads();
+            const u64 of = lane < nwarps ? *(volatile u64 *)&s_best[lane] : ~0ull;
+            int rank = 0;
+            for (int w = 0; w < nwarps; w++) {
+                const u64 x = __shfl_sync(FULL, of, w);
+                rank += x < of || (x == of && w < lane);
+            }
+            pass = __shfl_sync(FULL, of, __ffs(__ballot_sync(FULL, lane < nwarps && rank == K - 1)) - 1);
         }
 #pragma unroll
         for (int j = 0; j < TR; j++) {
-            bool want = row[j] != ~0u && (!full || code_less(cp[j], cs[j], tp, ts));
-            unsigned m;
-            while ((m = __ballot_sync(FULL, want))) {
-                const int src = __ffs(m) - 1;
-                const u64 p = __shfl_sync(FULL, cp[j], src), s = __shfl_sync(FULL, cs[j], src);
-                const u32 id = __shfl_sync(FULL, row[j], src);
-                warp_list_insert(mine, K, p, s, id);
-                tp = __shfl_sync(FULL, mine.p, K - 1);
-                ts = __shfl_sync(FULL, mine.s, K - 1);
-                full = __shfl_sync(FULL, mine.id, K - 1) != ~0u;
-                if (lane == src) want = false;
-                want = want && (!full || code_less(cp[j], cs[j], tp, ts));
+            const u64 bound = min(pass, (u64) * (volatile unsigned long long *)&s_bound);
+            bool want = c[j].id != ~0u && prim[j] <= bound && (!full || prim[j] <= tp);
+            if (!__any_sync(FULL, want)) continue;
+            if (want) {  // its keys too
+                topn_code(A, c[j].id, c[j].p, c[j].s);
+                want = !full || code_less(c[j].p, c[j].s, tp, ts);
             }
+            unsigned m = __ballot_sync(FULL, want);
+            if (!m) continue;
+            if (__popc(m) > 4) {
+                if (!want) c[j] = TopItem{~0ull, ~0ull, ~0u};
+                warp_sort(c[j]);
+                warp_list_merge(mine, c[j], K);
+                m = 0;
+            }
+            while (m) {
+                const int src = __ffs(m) - 1;
+                m &= m - 1;
+                warp_list_insert(mine, K, __shfl_sync(FULL, c[j].p, src), __shfl_sync(FULL, c[j].s, src),
+                                 __shfl_sync(FULL, c[j].id, src));
+            }
+            tp = __shfl_sync(FULL, mine.p, K - 1);
+            ts = __shfl_sync(FULL, mine.s, K - 1);
+            full = __shfl_sync(FULL, mine.id, K - 1) != ~0u;
+            if (full && lane == 0 && tp < bound) atomicMin(&s_bound, (unsigned long long)tp);
         }
     }
-    s_list[warp][lane] = mine;
-    __syncthreads();
+    for (int d = nwarps / 2; d; d >>= 1) {
+        s_list[warp][lane] = mine;
+        __syncthreads();
+        if (warp < d) warp_list_merge(mine, s_list[warp + d][lane], K);
+        __syncthreads();
+    }
     if (warp == 0) {
-        TopItem best{~0ull, ~0ull, ~0u};
-        u64 bp = ~0ull, bs = ~0ull;
-        bool bfull = false;
-        for (int w = 0; w < nwarps; w++) {
-            const TopItem c = s_list[w][lane];
-            bool want = lane < K && c.id != ~0u && (!bfull || code_less(c.p, c.s, bp, bs));
-            unsigned m;
-            while ((m = __ballot_sync(FULL, want))) {
-                const int src = __ffs(m) - 1;
-                const u64 p = __shfl_sync(FULL, c.p, src), s = __shfl_sync(FULL, c.s, src);
-                const u32 id = __shfl_sync(FULL, c.id, src);
-                warp_list_insert(best, K, p, s, id);
-                bp = __shfl_sync(FULL, best.p, K - 1);
-                bs = __shfl_sync(FULL, best.s, K - 1);
-                bfull = __shfl_sync(FULL, best.id, K - 1) != ~0u;
-                if (lane == src) want = false;
-                want = want && (!bfull || code_less(c.p, c.s, bp, bs));
-            }
-        }
-        if (lane < K) out_ids[(u64)blockIdx.x * K + lane] = best.id;
-        const unsigned have = __ballot_sync(FULL, lane < K && best.id != ~0u);
+        if (lane < K) out_ids[(u64)blockIdx.x * K + lane] = mine.id;
+        const unsigned have = __ballot_sync(FULL, lane < K && mine.id != ~0u);
         if (lane == 0) out_n[blockIdx.x] = (u32)__popc(have);
     }
 }
@@ -1875,14 +1968,14 @@ static gb_status run_topn(gb_agg *h, cudaStream_t st) {
     const bool small = K <= 32 && h->topn_small;  // warp-register lists
     {
         ProfScope ps(h, "k_topn", st);
-        if (small) k_topn_small<<<grid, 512, 0, st>>>(A, nullptr, n, (u32 *)h->topn_ids_a.p, (u32 *)h->topn_cnt.p);
+        if (small) k_topn_small<<<grid, 512, 0, st>>>(A, nullptr, n, 1, (u32 *)h->topn_ids_a.p, (u32 *)h->topn_cnt.p);
         else k_topn<<<grid, 512, smem, st>>>(A, nullptr, n, (u32 *)h->topn_ids_a.p, (u32 *)h->topn_cnt.p, sortn);
     }
     h->launches++;
     GB_CUDA(cudaGetLastError());
     // second pass over the grid*K candidate ids (padding ids are skipped)
     if (small)
-        k_topn_small<<<1, 512, 0, st>>>(A, (const u32 *)h->topn_ids_a.p, (u64)grid * K, (u32 *)h->topn_ids_b.p,
+        k_topn_small<<<1, 512, 0, st>>>(A, (const u32 *)h->topn_ids_a.p, (u64)grid * K, grid, (u32 *)h->topn_ids_b.p,
                                         (u32 *)h->topn_cnt.p);
     else
         k_topn<<<1, 512, smem, st>>>(A, (const u32 *)h->topn_ids_a.p, (u64)grid * K, (u32 *)h->topn_ids_b.p,

@@ -1,11 +1,12 @@
 """The radix pipeline's DOUBLE-sum tables on both sides of the estimate where
-their size changes, empty and full partitions and CTAs of several partitions."""
+their size changes, empty and full partitions and CTAs of several partitions;
+the register TopN against the general one."""
 import numpy as np
 import pytest
 
 import oracle
 from slothdb_gb300 import capi
-from slothdb_gb300.capi import BIGINT, DOUBLE
+from slothdb_gb300.capi import BIGINT, DOUBLE, SMALLINT
 from util import compare, gpu_to_dict
 
 pytestmark = [pytest.mark.gpu, pytest.mark.usefixtures("oracle_lib", "gblib")]
@@ -43,3 +44,25 @@ def test_double_sum_tables(est, groups):
     got = gpu_to_dict(result(types, [0], aggs, [k, x], est, runs=2), 1, out)
     compare(got, oracle.run_query(types, [0], aggs, [k, x]))
 
+
+@pytest.mark.parametrize("limit", [1, 2, 10, 15, 16, 17, 31, 32])
+@pytest.mark.parametrize("groups", [1, 9, 33, 4097, 200_000])
+def test_topn_lists_equal_the_general_path(limit, groups):
+    """Ties in the order column, NULLs among it, both directions, every type."""
+    rng = np.random.default_rng(groups + limit)
+    n = 2 * groups + 77
+    k = (rng.integers(0, groups, n) - groups // 2).astype(np.int64)
+    v = rng.integers(-40, 40, n)
+    x = np.round(rng.normal(0, 3, n))
+    s = rng.integers(-9, 9, n).astype(np.int16)
+    types = [BIGINT, BIGINT, DOUBLE, SMALLINT]
+    aggs = [("count_star", -1), ("sum", 1), ("max", 2), ("min", 3)]
+    nulls = [None, rng.random(n) < 0.4, rng.random(n) < 0.4, rng.random(n) < 0.4]
+    for col in range(1, 5):
+        for ascending in (False, True):
+            a, b = (result(types, [0], aggs, [k, v, x, s], groups, topn=(col, ascending, limit), nulls=nulls,
+                           options={"topn_small": small}) for small in (1, 0))
+            assert len(a) == len(b)
+            for p, q in zip(a, b):
+                for u, w in zip(p, q):
+                    np.testing.assert_array_equal(np.asarray(u), np.asarray(w))
