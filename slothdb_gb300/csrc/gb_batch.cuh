@@ -61,12 +61,14 @@ __device__ __forceinline__ void copy_words(void *dst, const void *src, int bytes
     for (int i = threadIdx.x; i < bytes / 4; i += blockDim.x) d[i] = s[i];
 }
 
-// Item (q, idx) covers words [idx * 65536, (idx+1) * 65536) of the query's
-// init range: the table words, then the validity words of every output column
+// Item (q, idx) covers words [idx * INIT_WORDS, (idx+1) * INIT_WORDS) of the
+// query's init range (a block's chain of stores bounds a small batch: 14
+// tables of up to 16,384 slots in items of 65,536 words 65 us, this 13): the table words, then the validity words of every output column
 // (all ones; the emit clears the bits of NULL results), then (COUNT(DISTINCT))
 // the pair sets, their NULL-key twins and the pair counters, after, for a VARCHAR
 // key the dictionary's hash slots (free), ref slots (unpublished) and its
 // eight counter words (zero).
+#define INIT_WORDS 4096
 __global__ void k_batch_init(const BQuery *qs, const BItem *items, u32 n_items) {
     for (u32 it = blockIdx.x; it < n_items; it += gridDim.x) {
         const BItem w = items[it];
@@ -79,11 +81,12 @@ __global__ void k_batch_init(const BQuery *qs, const BItem *items, u32 n_items) 
         const u64 sw = q.P.n_dist ? (q.P.dmask + 1) * (q.P.dnarrow ? 1 : 2) * (u64)q.P.n_dist : 0;
         const u64 nw = q.P.null_sets ? sw : 0;
         const u64 dempty = q.P.dnarrow ? ~0ull : EMPTY_KEY;
-        const u64 lo = (u64)w.idx * 65536, hi = min(q.init_words, lo + 65536);
+        const u64 lo = (u64)w.idx * INIT_WORDS, hi = min(q.init_words, lo + INIT_WORDS);
+        const u64 ns = (q.T.cap + 2) * (u64)stride;
+        const u32 wd0 = (u32)(lo % (u64)stride);  // state word of the item's first word
         for (u64 i = lo + threadIdx.x; i < hi; i += blockDim.x) {
             if (i < n0) {
-                const u64 ns = (q.T.cap + 2) * (u64)stride;
-                const int wd = (int)(i % (u64)stride);
+                const int wd = (int)((wd0 + (u32)(i - lo)) % (u32)stride);
                 if (i >= ns) q.T.keys[i - ns] = EMPTY_KEY;
                 else q.T.states[i] = wd < q.P.words ? q.P.word_init[wd] : 0;
             } else if (i < n1) {
@@ -1106,7 +1109,7 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
             const u64 sw = (h->plan.dmask + 1) * (h->plan.dnarrow ? 1 : 2) * (u64)h->plan.n_dist;
             d.init_words += sw * (h->plan.null_sets ? 2 : 1) + 2 + GB_MAX_DISTINCT;
         }
-        for (u64 c = 0; c * 65536 < d.init_words; c++) it_init.push_back({q, (u32)c});
+        for (u64 c = 0; c * INIT_WORDS < d.init_words; c++) it_init.push_back({q, (u32)c});
         d.tile_rows = b->tile_rows;
         for (u64 c = 0; c * b->tile_rows < n; c++) it_ing.push_back({q, (u32)c});
         for (u64 c = 0; c * (COMPACT_PER * 256) < h->cap + 2; c++) it_cmp.push_back({q, (u32)c});
