@@ -24,12 +24,13 @@
 //               Partition regions have per-partition capacities; a region
 //               that overflows is grown (and its tuples moved) by the host,
 //               and a re-execution keeps the grown capacities.
-//   P2 agg:     one CTA per partition: a shared open-addressing table (keys,
+//   P2 agg:     a CTA per partition: a shared open-addressing table (keys,
 //               32-bit counts) with either the state words beside it and a
 //               warp pre-combine of equal keys (32-bit hash match checked on
 //               the full key), or, when every op is a DOUBLE SUM, the words
-//               in the partition's L2 slice folded tuple by tuple as L2
-//               reductions; a table that overflows folds the rest into the
+//               in the CTA's L2 slice folded tuple by tuple as L2 reductions
+//               (persistent CTAs, each with one slice for all of its
+//               partitions); a table that overflows folds the rest into the
 //               HBM hash table.
 //   P3 hot:     per-CTA hot partials are reduced in a fixed order and
 //               emitted.  (DOUBLE sums are exact to rounding but, as with any
@@ -965,17 +966,7 @@ __global__ void __launch_bounds__(RADIX_BLOCK, 1)
     if (threadIdx.x == 0 && s_new) atomicAdd(&T.ctl->n_groups, s_new);
 }
 
-// P2 for plans whose ops are all DOUBLE SUMs of the one value column (the
-// COUNT / SUM / AVG(DOUBLE) shape): shared memory holds only keys and u32
-// counts; the sum words live in the CTA's slice of p2_words and fold as
-// fire-and-forget L2 reductions.  The slot comes from bits 20.. of the P1 hash
-// (the partition took its top bits).  A CTA takes partitions blockIdx,
-// blockIdx + grid, ..., so its slice stays in L2; the emit leaves the slots
-// that it reads empty for the next partition, whose tuples head for L2
-// meanwhile.  Two CTAs share an SM where tables of half the size hold the
-// estimate: one probes while the other divides and writes.  28.5M tuples of
-// 6.2M groups, tables of 8192 slots: 739 -> 510 us (717 with the words of one
-// round of slots read at a time: the emit waited for L2).
+// A tuple whose table is full.
 template <int NOPS>
 __device__ __noinline__ void p2_sum_overflow(const Plan &P, const TableRef &T, u64 pk, u64 x, u32 *new_groups) {
     u64 v[NOPS];
@@ -1000,6 +991,17 @@ __device__ __forceinline__ u32 p2_walk(u64 *keys, int SP, int probe, u32 s, u64 
     return (u32)SP;
 }
 
+// P2 for plans whose ops are all DOUBLE SUMs of the one value column (the
+// COUNT / SUM / AVG(DOUBLE) shape): shared memory holds only keys and u32
+// counts; the sum words live in the CTA's slice of p2_words and fold as
+// fire-and-forget L2 reductions.  The slot comes from bits 20.. of the P1 hash
+// (the partition took its top bits).  A CTA takes partitions blockIdx,
+// blockIdx + grid, ..., so its slice stays in L2; the emit leaves the slots
+// that it reads empty for the next partition, whose tuples head for L2
+// meanwhile.  Two CTAs share an SM where tables of half the size hold the
+// estimate: one probes while the other divides and writes.  28.5M tuples of
+// 6.2M groups, tables of 8192 slots: 739 -> 510 us (717 with the words of one
+// round of slots read at a time: the emit waited for L2).
 template <int NOPS>
 __global__ void __launch_bounds__(RADIX_BLOCK, 1)
     k_part_agg_sum(const __grid_constant__ Plan P, const __grid_constant__ RadixPlan R, const RadixRef X,
@@ -1253,7 +1255,9 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
     if (P.words > GB_MAX_WORDS) return GB_ERR_UNSUPPORTED;
     R.spec = p1_spec(P, R, nullable_mask);
     // P2: one shared table of `sub` slots per partition (keys + counts only,
-    // 12 bytes a slot, when the state words fold in L2)
+    // 12 bytes a slot, when the state words fold in L2: 8192 slots let two
+    // CTAs share an SM, 717 us against 739 with one of 16384 in a first form;
+    // an estimate beyond 4096 such partitions takes the larger table)
     int sp = 8192;
     R.sub = sp;
     const u64 max_np = 4096;

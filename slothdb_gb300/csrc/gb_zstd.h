@@ -8,9 +8,10 @@
 // state machines from one backward bit stream, tables predefined, RLE,
 // described in the block, or repeated; three repeat offsets).
 //
-// Header-only and __host__ __device__: the page inflate runs it on one lane
-// per page; the same code built for the host is what the CPU tests check
-// against another implementation.  Every read and write is bounds-checked
+// Header-only and __host__ __device__: the page inflate builds its tables with
+// it and decodes on one lane the pages that its block of threads does not take
+// (gb_inflate.cuh); the same code built for the host is what the CPU tests
+// check against another implementation.  Every read and write is bounds-checked
 // against the source, the destination and the scratch: a malformed frame
 // returns -1, never a read or write outside them.
 #pragma once
