@@ -62,12 +62,13 @@ __device__ __forceinline__ void copy_words(void *dst, const void *src, int bytes
 }
 
 // Item (q, idx) covers words [idx * INIT_WORDS, (idx+1) * INIT_WORDS) of the
-// query's init range (a block's chain of stores bounds a small batch: 14
-// tables of up to 16,384 slots in items of 65,536 words 65 us, this 13): the table words, then the validity words of every output column
-// (all ones; the emit clears the bits of NULL results), then (COUNT(DISTINCT))
-// the pair sets, their NULL-key twins and the pair counters, after, for a VARCHAR
-// key the dictionary's hash slots (free), ref slots (unpublished) and its
-// eight counter words (zero).
+// query's init range: the table words, then the validity words of every output
+// column (all ones; the emit clears the bits of NULL results), then
+// (COUNT(DISTINCT)) the pair sets, their NULL-key twins and the pair counters,
+// after, for a VARCHAR key the dictionary's hash slots (free), ref slots
+// (unpublished) and its eight counter words (zero).  A block's chain of stores
+// bounds a small batch: 14 tables of up to 16,384 slots 65 us in items of 65,536
+// words, 13 in these.
 #define INIT_WORDS 4096
 __global__ void k_batch_init(const BQuery *qs, const BItem *items, u32 n_items) {
     for (u32 it = blockIdx.x; it < n_items; it += gridDim.x) {
