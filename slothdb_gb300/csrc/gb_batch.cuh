@@ -172,9 +172,9 @@ __device__ __forceinline__ void fast_apply_global(const FastPlan &F, u64 *w, u64
 }
 
 // Narrow shared states: count u32; ADD as a (lo, hi) u32 pair with carry;
-// CNT_NN u32; MIN/MAX s32 over SMALLINT/INTEGER, s64 over BIGINT and (order
-// preserving) DOUBLE; a DOUBLE sum is a double.  Every update is a native
-// 32-bit shared atomic except the 64-bit MIN/MAX and the DOUBLE sum.
+// CNT_NN and OP_DIST u32; MIN/MAX s32 over SMALLINT/INTEGER, s64 over BIGINT
+// and (order preserving) DOUBLE; a DOUBLE sum is a double.  Every update is a
+// native 32-bit shared atomic except the 64-bit MIN/MAX and the DOUBLE sum.
 template <int NOPS, bool FLT>
 __device__ __forceinline__ void fast_apply_smem(const FastPlan &F, u32 *st, u64 cnt, const u64 *v) {
     atomicAdd(st, (u32)cnt);
@@ -201,11 +201,11 @@ __device__ __forceinline__ void fast_apply_smem(const FastPlan &F, u32 *st, u64 
             if (wide) atomicMax((long long *)w, (long long)v[i]);
             else atomicMax((int *)w, (int)(i64)v[i]);
             break;
-        default:  // CNT_NN, the DOUBLE ops
-            if (!FLT || kind == OP_CNT_NN) atomicAdd(w, (u32)v[i]);
-            else if (kind == OP_ADD_F) atomicAdd((double *)w, __longlong_as_double((i64)v[i]));
-            else if (kind == OP_MIN_F) atomicMin((long long *)w, (long long)v[i]);
-            else atomicMax((long long *)w, (long long)v[i]);
+        default:  // the DOUBLE ops (64-bit words); counts (CNT_NN, OP_DIST) add in 32 bits, as op_apply adds what it does not name
+            if (FLT && kind == OP_ADD_F) atomicAdd((double *)w, __longlong_as_double((i64)v[i]));
+            else if (FLT && kind == OP_MIN_F) atomicMin((long long *)w, (long long)v[i]);
+            else if (FLT && kind == OP_MAX_F) atomicMax((long long *)w, (long long)v[i]);
+            else atomicAdd(w, (u32)v[i]);
             break;
         }
     }
