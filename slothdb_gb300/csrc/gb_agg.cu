@@ -97,7 +97,7 @@ struct IngestArgs {
     u32 first_tile;
     int32_t smem_slots;
     int32_t smem_probe;
-    int32_t pad;
+    int32_t match_least;  // k_ingest_fast's WarpMatch (plans with DOUBLE or COUNT(DISTINCT) ops)
 };
 
 // Persistent ingest: CTAs claim tiles of rows until none are left or the
@@ -1186,7 +1186,7 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
         A.n_tiles = (u32)(n_tiles_total - first);
         A.smem_slots = S;
         A.smem_probe = h->smem_probe;
-        A.pad = 0;
+        A.match_least = 0;
         TableRef T = table_ref(h);
         int g = (int)std::min<u64>((u64)grid, n_tiles_total - first);
         if (fast) {

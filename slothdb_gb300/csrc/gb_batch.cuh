@@ -385,11 +385,23 @@ __device__ __forceinline__ int fast_key_of(u32 kd, i64 a_, i64 b_, u32 vbits, u6
     return 0;
 }
 
+// Whether a warp combines its equal keys before it folds them (MATCH_ASK): it
+// looks at every MATCH_EVERY-th of its steps and goes by the rows of the key
+// that most lanes of that step had.
+enum { MATCH_NO, MATCH_YES, MATCH_ASK };
+#define MATCH_EVERY 32
+struct WarpMatch {
+    int least;     // such rows from which on the warp combines (0: always, above 32: never)
+    int left;      // steps until it looks again
+    bool on;
+    __device__ __forceinline__ WarpMatch(int n) : least(n), left(n > 32 ? 0x7fffffff : 0), on(n == 0) {}
+};
+
 // One warp step of the fast path on fetched rows.
-template <bool PRECOMBINE, int NOPS, bool FILT, bool FLT, bool SPILL = false, bool DIST = false>
+template <int MATCH, int NOPS, bool FILT, bool FLT, bool SPILL = false, bool DIST = false>
 __device__ __forceinline__ void fast_rows(const FastPlan &F, const FastFilters &FF, const TableRef &T, u64 *keys,
                                           u32 *st, int S, const FastRaw<NOPS, FILT> &w, u32 *new_groups,
-                                          const Plan *SP = nullptr, u32 *new_pairs = nullptr) {
+                                          const Plan *SP = nullptr, u32 *new_pairs = nullptr, WarpMatch *M = nullptr) {
     const int lane = threadIdx.x & 31;
     bool act = w.act && (!FILT || fast_pass(F, FF, w.f, w.vbits));
     u64 pk = 0;
@@ -420,9 +432,18 @@ __device__ __forceinline__ void fast_rows(const FastPlan &F, const FastFilters &
     const unsigned am = __ballot_sync(FULL, act);
     if (am == 0) return;
     u64 cnt = 1;
-    if (PRECOMBINE) {
+    bool match = MATCH != MATCH_NO, look = false;
+    if (MATCH == MATCH_ASK) {
+        look = M->left-- == 0;
+        match = M->on || look;
+    }
+    if (match) {
         const unsigned peers = __match_any_sync(FULL, pk) & am;
         const bool leader = act && ((__ffs(peers) - 1) == lane);
+        if (look) {
+            M->on = (int)__reduce_max_sync(FULL, (unsigned)__popc(peers)) >= M->least;
+            M->left = MATCH_EVERY - 1;
+        }
         unsigned rem = leader ? (peers & ~(1u << lane)) : 0u;
         cnt = __popc(peers);
         const int maxit = __reduce_max_sync(FULL, (unsigned)__popc(rem));
@@ -490,7 +511,7 @@ __device__ __forceinline__ void fast_tile(const FastPlan &F, const FastFilters &
     fast_fetch<NOPS, NULLS, FILT>(F, FF, base + (threadIdx.x & 31), t1, cur);
     for (; base < t1; base += step) {
         fast_fetch<NOPS, NULLS, FILT>(F, FF, base + step + (threadIdx.x & 31), t1, nxt);
-        fast_rows<PRECOMBINE, NOPS, FILT, false>(F, FF, T, keys, st, S, cur, new_groups);
+        fast_rows<PRECOMBINE ? MATCH_YES : MATCH_NO, NOPS, FILT, false>(F, FF, T, keys, st, S, cur, new_groups);
         cur = nxt;
     }
     __syncthreads();
@@ -878,7 +899,7 @@ static FastPlan make_fast_plan(const Plan &P, FastFilters &FF, int max_ops = BAT
 // query's tiles, with one narrow shared table per CTA for the whole launch
 // and spill records instead of re-runs.  Same tile-claim / spill-threshold
 // protocol as k_ingest, so run_ingest drives both.
-template <bool PRE, int NOPS, bool NULLS, bool FILT, bool FLT = false, bool DIST = false>
+template <int MATCH, int NOPS, bool NULLS, bool FILT, bool FLT = false, bool DIST = false>
 __global__ void __launch_bounds__(512, 2)
     k_ingest_fast(const __grid_constant__ Plan P, const __grid_constant__ FastPlan F,
                   const __grid_constant__ FastFilters FF, const TableRef T, const IngestArgs A) {
@@ -898,6 +919,7 @@ __global__ void __launch_bounds__(512, 2)
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 step = (u64)(blockDim.x >> 5) * 32;
+    WarpMatch M(A.match_least);
     for (int at = 0;; at ^= 1) {
         const u32 t = s_tile[at];
         if (t >= A.n_tiles) break;
@@ -909,7 +931,7 @@ __global__ void __launch_bounds__(512, 2)
         fast_fetch<NOPS, NULLS, FILT>(F, FF, base + lane, t1, cur);
         for (; base < t1; base += step) {
             fast_fetch<NOPS, NULLS, FILT>(F, FF, base + step + lane, t1, nxt);
-            fast_rows<PRE, NOPS, FILT, FLT, true, DIST>(F, FF, T, keys, st, S, cur, &s_new, &P, &s_pairs);
+            fast_rows<MATCH, NOPS, FILT, FLT, true, DIST>(F, FF, T, keys, st, S, cur, &s_new, &P, &s_pairs, &M);
             cur = nxt;
         }
         if (threadIdx.x == 0 && *(volatile u32 *)&T.ctl->spill_count > T.spill_threshold)
@@ -933,16 +955,13 @@ typedef void (*FastIngestKernel)(Plan, FastPlan, FastFilters, TableRef, IngestAr
         }                                                                                       \
     }
 
-// Plans with DOUBLE ops: one kernel for each number of ops, with the NULL and
-// predicate code whether they need it or not.
-static FastIngestKernel fast_ingest_kernel_f(int pre, int nops) {
-    static const FastIngestKernel tab[2][FAST_MAX_OPS] = {
-        {k_ingest_fast<false, 1, true, true, true>, k_ingest_fast<false, 2, true, true, true>,
-         k_ingest_fast<false, 3, true, true, true>, k_ingest_fast<false, 4, true, true, true>},
-        {k_ingest_fast<true, 1, true, true, true>, k_ingest_fast<true, 2, true, true, true>,
-         k_ingest_fast<true, 3, true, true, true>, k_ingest_fast<true, 4, true, true, true>},
-    };
-    return tab[pre][nops - 1];
+// Plans with DOUBLE ops: one kernel for each number of ops, with the NULL,
+// predicate and key match code whether they need it or not.
+static FastIngestKernel fast_ingest_kernel_f(int nops) {
+    static const FastIngestKernel tab[FAST_MAX_OPS] = {
+        k_ingest_fast<MATCH_ASK, 1, true, true, true>, k_ingest_fast<MATCH_ASK, 2, true, true, true>,
+        k_ingest_fast<MATCH_ASK, 3, true, true, true>, k_ingest_fast<MATCH_ASK, 4, true, true, true>};
+    return tab[nops - 1];
 }
 
 // Plans with COUNT(DISTINCT), likewise (with and without DOUBLE ops): 20M rows,
@@ -950,18 +969,18 @@ static FastIngestKernel fast_ingest_kernel_f(int pre, int nops) {
 // bound by the pair set's compare-and-swaps, which miss L2 (512 MB).
 static FastIngestKernel fast_ingest_kernel_d(int flt, int nops) {
     static const FastIngestKernel tab[2][FAST_MAX_OPS] = {
-        {k_ingest_fast<false, 1, true, true, false, true>, k_ingest_fast<false, 2, true, true, false, true>,
-         k_ingest_fast<false, 3, true, true, false, true>, k_ingest_fast<false, 4, true, true, false, true>},
-        {nullptr, k_ingest_fast<false, 2, true, true, true, true>, k_ingest_fast<false, 3, true, true, true, true>,
-         k_ingest_fast<false, 4, true, true, true, true>},
+        {k_ingest_fast<MATCH_ASK, 1, true, true, false, true>, k_ingest_fast<MATCH_ASK, 2, true, true, false, true>,
+         k_ingest_fast<MATCH_ASK, 3, true, true, false, true>, k_ingest_fast<MATCH_ASK, 4, true, true, false, true>},
+        {nullptr, k_ingest_fast<MATCH_ASK, 2, true, true, true, true>, k_ingest_fast<MATCH_ASK, 3, true, true, true, true>,
+         k_ingest_fast<MATCH_ASK, 4, true, true, true, true>},
     };
     return tab[flt][nops - 1];
 }
 
 static FastIngestKernel fast_ingest_kernel(int pre, int nops, int nulls, int filt) {
     static const FastIngestKernel tab[2][FAST_MAX_OPS + 1][2][2] = {
-        {GB_FI4(false, 0), GB_FI4(false, 1), GB_FI4(false, 2), GB_FI4(false, 3), GB_FI4(false, 4)},
-        {GB_FI4(true, 0), GB_FI4(true, 1), GB_FI4(true, 2), GB_FI4(true, 3), GB_FI4(true, 4)},
+        {GB_FI4(MATCH_NO, 0), GB_FI4(MATCH_NO, 1), GB_FI4(MATCH_NO, 2), GB_FI4(MATCH_NO, 3), GB_FI4(MATCH_NO, 4)},
+        {GB_FI4(MATCH_YES, 0), GB_FI4(MATCH_YES, 1), GB_FI4(MATCH_YES, 2), GB_FI4(MATCH_YES, 3), GB_FI4(MATCH_YES, 4)},
     };
     return tab[pre][nops][nulls][filt];
 }
@@ -981,8 +1000,15 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
     const int S = h->est_groups <= (u64)A.smem_slots ? A.smem_slots : 0;
     // narrow shared atomics beat the warp key match; without a shared table,
     // few groups mean hot HBM slots, which the match relieves
-    const bool pre = h->precombine_set ? h->precombine
-                                       : (S == 0 ? h->est_groups <= 4096 : F.sums_f && h->est_groups <= FAST_PRE_F);
+    const bool pre = h->precombine_set ? h->precombine : S == 0 && h->est_groups <= 4096;
+    // with DOUBLE or COUNT(DISTINCT) ops the warps see for themselves whether
+    // their rows share keys: a hot key's rows meet in turn in an HBM slot, or in
+    // the compare-and-swap loop of a DOUBLE sum in shared memory (its other ops
+    // are native there and take no match).  Calls of 4M rows, SUM(DOUBLE), never
+    // / always / as the warps see: 64 groups uniform 120 / 131 / 118 us, Zipf(1.1)
+    // 761 / 142 / 155; 300,000 groups uniform 129 / 153 / 130, one key in every
+    // other row 4,134 / 424 / 426; COUNT(DISTINCT) of the last 2,381 / 601 / 602
+    A.match_least = h->precombine_set ? (h->precombine ? 0 : 33) : (S == 0 ? MATCH_HBM : (F.sums_f ? MATCH_SHARED : 33));
     A.smem_slots = S;
     const size_t smem = FAST_SMEM(S, F.swords);
     static bool attr_set = false;
@@ -993,10 +1019,9 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
                     for (int f = 0; f < 2; f++)
                         GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel(a, n, u, f),
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        for (int a = 0; a < 2; a++)
-            for (int n = 1; n <= FAST_MAX_OPS; n++)
-                GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel_f(a, n), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024));
+        for (int n = 1; n <= FAST_MAX_OPS; n++)
+            GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel_f(n), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         200 * 1024));
         for (int f = 0; f < 2; f++)
             for (int n = 1 + f; n <= FAST_MAX_OPS; n++)
                 GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel_d(f, n), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1006,7 +1031,7 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
     {
         ProfScope ps(h, "k_ingest_fast", st);
         const FastIngestKernel k = F.dist ? fast_ingest_kernel_d(F.flt, F.n_ops)
-                                   : F.flt ? fast_ingest_kernel_f(pre, F.n_ops)
+                                   : F.flt ? fast_ingest_kernel_f(F.n_ops)
                                            : fast_ingest_kernel(pre, F.n_ops, F.nulls != 0, F.n_filters != 0);
         k<<<grid, 512, smem, st>>>(h->plan, F, X.FF, T, A);
     }

@@ -587,10 +587,11 @@ __device__ __forceinline__ void compact_chunk(const Plan &P, const EmitArgs &E, 
 #define FAST_MAX_FILTERS 2
 // shared memory of a CTA's table of S slots: keys, states, two out-of-band states
 #define FAST_SMEM(S, swords) ((size_t)(S) * 8 + ((size_t)(S) + 2) * 4 * (size_t)(swords))
-// with a DOUBLE sum in shared memory (a compare-and-swap loop), a warp's equal
-// keys are combined first for up to so many estimated groups (3M rows: 3
-// groups 106 us with, 303 without; 64 groups 77 and 65 us)
-#define FAST_PRE_F 24
+// rows of one key in a warp's step from which on the warp combines equal keys
+// before the fold: of a DOUBLE sum in shared memory, of any op in HBM (figures
+// at the rule, launch_ingest_fast)
+#define MATCH_SHARED 4
+#define MATCH_HBM 2
 
 // Plan description kept in registers by the fast tile path (up to
 // FAST_MAX_FILTERS predicates on integer or DOUBLE columns; keys SINGLE /
