@@ -975,20 +975,35 @@ __device__ __noinline__ void p2_sum_overflow(const Plan &P, const TableRef &T, u
     global_fold_n<NOPS>(P, T, pk, 1, v, new_groups);
 }
 
-// The slot of pk past home slot s, which holds another key (SP: none within `probe`).
-__device__ __forceinline__ u32 p2_walk(u64 *keys, int SP, int probe, u32 s, u64 pk) {
+// The slots of the tuples t past their home slots `at`, which hold the keys k
+// (SP: none within `probe`); the tuples of a thread go on side by side.
+__device__ __forceinline__ void p2_walk(u64 *keys, int SP, int probe, u32 *at, const u64 *k, const ulonglong2 *t) {
     volatile u64 *vk = keys;
+    bool open[P2_ROWS], any = false;
+#pragma unroll
+    for (int j = 0; j < P2_ROWS; j++) any |= open[j] = k[j] != t[j].x && t[j].x != EMPTY_KEY;
 #pragma unroll 1
-    for (int q = 1; q < probe; q++) {
-        s = (s + 1) & (u32)(SP - 1);
-        u64 k = vk[s];
-        if (k == EMPTY_KEY) {
-            const u64 old = atomicCAS(&keys[s], EMPTY_KEY, pk);
-            k = (old == EMPTY_KEY) ? pk : old;
+    for (int q = 1; any && q < probe; q++) {
+        u64 x[P2_ROWS];
+        any = false;
+#pragma unroll
+        for (int j = 0; j < P2_ROWS; j++) {
+            if (open[j]) at[j] = (at[j] + 1) & (u32)(SP - 1);
+            x[j] = open[j] ? vk[at[j]] : t[j].x;
         }
-        if (k == pk) return s;
+#pragma unroll
+        for (int j = 0; j < P2_ROWS; j++) {
+            if (x[j] == EMPTY_KEY && open[j]) {
+                const u64 old = atomicCAS(&keys[at[j]], EMPTY_KEY, t[j].x);
+                x[j] = (old == EMPTY_KEY) ? t[j].x : old;
+            }
+            open[j] = open[j] && x[j] != t[j].x;
+            any |= open[j];
+        }
     }
-    return (u32)SP;
+#pragma unroll
+    for (int j = 0; j < P2_ROWS; j++)
+        if (open[j]) at[j] = (u32)SP;
 }
 
 // P2 for plans whose ops are all DOUBLE SUMs of the one value column (the
@@ -1059,9 +1074,7 @@ __global__ void __launch_bounds__(RADIX_BLOCK, 1)
                 const u64 old = atomicCAS(&keys[at[j]], EMPTY_KEY, t[j].x);
                 k[j] = (old == EMPTY_KEY) ? t[j].x : old;
             }
-#pragma unroll
-            for (int j = 0; j < P2_ROWS; j++)
-                if (k[j] != t[j].x && t[j].x != EMPTY_KEY) at[j] = p2_walk(keys, SP, R.agg_probe, at[j], t[j].x);
+            p2_walk(keys, SP, R.agg_probe, at, k, t);
             __syncwarp();  // the lanes' atomics go out together, however long each probed
 #pragma unroll
             for (int j = 0; j < P2_ROWS; j++) {
@@ -1232,6 +1245,20 @@ int radix_spec_of(const Plan &P, const RadixPlan &R, u64 nullable_mask) { return
 static_assert(P2_SUB_MAX * 12 <= 224 * 1024 && 2 * (P2_SUB_MAX / 2 * 12 + 1024) <= 224 * 1024, "tables of k_part_agg_sum");
 static const size_t kSmemBudget = 224 * 1024;  // <= the 227 KiB opt-in minus static shared memory
 
+// k_part_agg_sum's tables, by the partitions that the plan ended with (the
+// generic P1 has room for 1,024): 8,192 slots, so that two CTAs share an SM,
+// where the estimate fills them to 7/8 at most, else 16,384 (7.3M groups of
+// INTEGER keys 1.01 ms a call small, ~1.15 large; 30M of BIGINT keys 3.28 and
+// 3.18; tables too small send groups through the HBM table: 11.5M of INTEGER
+// keys 3.80 ms small, 1.53 large).  P2_MIN_SMALL partitions or more: together
+// the small tables then hold what 64 large ones do, for an estimate that is
+// too low (900,000 groups, 100,000 estimated: 2.42 ms with 64 small ones, 0.73).
+static void radix_p2_table(const Plan &P, RadixPlan &R) {
+    if (!radix_p2_global_words(P, R)) return;
+    const u64 np = 1ull << R.pbits, small = P2_SUB_MAX / 2;
+    R.sub = np >= P2_MIN_SMALL && R.est <= np * (small * 7 / 8) ? (int)small : P2_SUB_MAX;
+}
+
 gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullable_mask) {
     memset(&R, 0, sizeof R);
     if (P.key_mode == KEY_STRING || P.n_dist) return GB_ERR_UNSUPPORTED;
@@ -1254,17 +1281,10 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
     }
     if (P.words > GB_MAX_WORDS) return GB_ERR_UNSUPPORTED;
     R.spec = p1_spec(P, R, nullable_mask);
-    // P2: one shared table of `sub` slots per partition (keys + counts only,
-    // 12 bytes a slot, when the state words fold in L2: 8192 slots let two
-    // CTAs share an SM, 717 us against 739 with one of 16384 in a first form;
-    // an estimate beyond 4096 such partitions takes the larger table)
+    // P2: one shared table of `sub` slots per partition
     int sp = 8192;
     R.sub = sp;
-    const u64 max_np = 4096;
-    if (radix_p2_global_words(P, R) && est_groups > max_np * (sp * 7 / 10)) {
-        sp = P2_SUB_MAX;
-        R.sub = sp;
-    }
+    R.est = est_groups;
     while (sp > 1024 && !radix_p2_global_words(P, R) && radix_p2_smem(P, R) > kSmemBudget) {
         sp /= 2;
         R.sub = sp;
@@ -1274,8 +1294,8 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
     R.p2_pre = radix_p2_global_words(P, R) ? 0 : 1;
     // partitions so that a partition's groups fill its table to <= ~0.7
     const u64 per_part = (u64)sp * 7 / 10;
-    u64 np = pow2_at_least(std::max<u64>((est_groups + per_part - 1) / per_part, 64));
-    np = std::min<u64>(np, max_np);
+    u64 np = pow2_at_least(std::max<u64>((est_groups + per_part - 1) / per_part, radix_p2_global_words(P, R) ? P2_MIN_SMALL : 64));
+    np = std::min<u64>(np, 4096);
     int pb = 0;
     while ((1ull << pb) < np) pb++;
     R.pbits = pb;
@@ -1285,7 +1305,10 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
     R.nh = 4096;
     R.nsup = 64;
     R.hot_probe = 8;
-    if (R.spec) return radix_p1d_smem(R) <= kSmemBudget ? GB_OK : GB_ERR_UNSUPPORTED;
+    if (R.spec) {
+        radix_p2_table(P, R);
+        return radix_p1d_smem(R) <= kSmemBudget ? GB_OK : GB_ERR_UNSUPPORTED;
+    }
     while (radix_p1_smem(P, R) > kSmemBudget) {
         // keep the hot set large (a key left out of it lands in P2, where its
         // repeats contend): shrink the warp-private tier first
@@ -1302,6 +1325,7 @@ gb_status radix_prepare(const Plan &P, RadixPlan &R, u64 est_groups, u64 nullabl
         } else if (R.pbits > 6) R.pbits--;
         else return GB_ERR_UNSUPPORTED;
     }
+    radix_p2_table(P, R);
     return GB_OK;
 }
 
@@ -1311,6 +1335,7 @@ gb_status radix_set_bits(const Plan &P, RadixPlan &R, int bits) {
     RadixPlan t = R;
     t.pbits = bits;
     if ((t.spec ? radix_p1d_smem(t) : radix_p1_smem(P, t)) > kSmemBudget) return GB_ERR_UNSUPPORTED;
+    radix_p2_table(P, t);
     R = t;
     return GB_OK;
 }

@@ -11,6 +11,7 @@
 #define REG_HOT 4     // hottest keys accumulated in per-lane registers
 #define RADIX_BLOCK 1024
 #define P2_SUB_MAX 16384  // slots of k_part_agg_sum's tables: one CTA per SM, or two of half the slots and threads
+#define P2_MIN_SMALL 128  // partitions from which on the tables may be of half the slots
 #define P2_EMIT 4     // rounds of 32 slots whose words are read together (k_part_agg_sum)
 #define P2_ROWS 2     // tuples of a thread in flight (k_part_agg_sum)
 #define CURSOR_PAD 32    // partition cursors 128 bytes apart (spread over L2 slices)
@@ -28,6 +29,7 @@ struct RadixPlan {
     int32_t nh;                         // hot keys (dense indices [0, nh))
     int32_t nsup;                       // super-hot keys: indices [0, nsup)
     int32_t sub;                        // P2 shared-table slots (power of two)
+    u64 est;                            // estimated groups
     int32_t wcb;                        // P1 write-combining tuples per partition
     int32_t hot_probe;
     int32_t agg_probe;
