@@ -1039,9 +1039,16 @@ static gb_status grow_and_merge(gb_agg *h, u64 new_cap, u32 pending, cudaStream_
             GB_CUDA(cudaMemsetAsync(&dctl->spill_count, 0, sizeof(u32), st));
             return GB_OK;
         }
-        // compact the re-spilled tail to the front
-        GB_CUDA(cudaMemcpyAsync(h->spill.p, (u64 *)h->spill.p + (size_t)pending * recw, (size_t)again * recw * 8,
-                                cudaMemcpyDeviceToDevice, st));
+        // compact the re-spilled tail to the front; where the two overlap (the
+        // rehash spilled too), by way of the old table, whose slots are read
+        const u64 *tail = (const u64 *)h->spill.p + (size_t)pending * recw;
+        const size_t bytes = (size_t)again * recw * 8;
+        if (again > pending) {
+            if ((s = h->table_old.ensure(bytes))) return s;
+            GB_CUDA(cudaMemcpyAsync(h->table_old.p, tail, bytes, cudaMemcpyDeviceToDevice, st));
+            tail = (const u64 *)h->table_old.p;
+        }
+        GB_CUDA(cudaMemcpyAsync(h->spill.p, tail, bytes, cudaMemcpyDeviceToDevice, st));
         pending = again;
         new_cap = h->cap * 2;
     }
