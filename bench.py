@@ -1121,7 +1121,7 @@ def run_parquet(args):
     raw = g.profile()
     prof = {k: vv[1] / max(1, vv[0]) for k, vv in raw.items()}
     # the page decode of a step: every launch of its kernels
-    inf_ms = sum(vv[1] for k, vv in raw.items() if k.startswith("k_pz_") or k == "k_pq_inflate")
+    inf_ms = sum(vv[1] for k, vv in raw.items() if k.startswith(("k_pz_", "k_pq_inflate")))
     g.set_profiling(False)
     clocks = Clocks(local)
     clocks.start()

@@ -411,7 +411,8 @@ __device__ __forceinline__ bool sn_piece(const uint8_t *src, const u32 slen, uin
             const u32 i = t + k * XT, tag = c[i], ty = tag & 3u;
             u32 cs = ty == 0 ? (tag >> 2) + 2 : 2 + ((0x310u >> (4 * (ty - 1))) & 15u);  // copies: 2, 3, 5 bytes
             if (tag >= 240 && ty == 0) cs = min(sn_decode(c + i).cs, 0x10000u);
-            jump[sn_at(i)] = (uint16_t)min(i + cs, 0xffffu);
+            // past the page's end: to the next segment, where all chains meet
+            jump[sn_at(i)] = (uint16_t)(i < avail ? min(i + cs, 0xffffu) : (i | 63) + 1);
         }
         __syncthreads();
 #pragma unroll
@@ -498,13 +499,12 @@ __device__ __forceinline__ bool sn_piece(const uint8_t *src, const u32 slen, uin
     return true;
 }
 
-// Stored and SNAPPY pieces: a block claims pieces from a counter (the word
-// after the last job, zero at launch), longest first, until none is left.
-__global__ void __launch_bounds__(XT, X_CTAS) k_pq_inflate(const uint8_t *__restrict__ file, InflateJob *jobs, uint32_t n,
-                                                      uint8_t *img, uint32_t *lvl, Ctl *ctl) {
+// Stored and SNAPPY pieces: a block claims pieces from a counter (zero at
+// launch), longest first, until none is left.
+__global__ void __launch_bounds__(XT, X_CTAS) k_pq_inflate(const uint8_t *__restrict__ file, const InflateJob *jobs,
+                                                      uint32_t n, uint32_t *next, uint8_t *img, uint32_t *lvl, Ctl *ctl) {
     extern __shared__ __align__(16) unsigned char x_smem[];
     SnapShared &S = *(SnapShared *)x_smem;
-    uint32_t *next = (uint32_t *)(jobs + n);
     for (;;) {
         if (threadIdx.x == 0) S.job = atomicAdd(next, 1u);
         __syncthreads();
@@ -521,6 +521,170 @@ __global__ void __launch_bounds__(XT, X_CTAS) k_pq_inflate(const uint8_t *__rest
             x_level(J, dst, !ok, lvl);
         }
         __syncthreads();  // S.job is written again
+    }
+}
+
+// Small pieces, where there are many, one warp each (k_pq_inflate_small): no
+// barriers, and 48 of them on an SM at once instead of one.  The warp decodes a round of elements at a time.  Lane L reads the 8
+// compressed bytes at ip + L (one aligned word per lane, redistributed by
+// shuffles) and decodes the element a tag there would be; the chain of real
+// tags from ip (each start plus its element's compressed size) is walked with
+// shuffles over the lanes' sizes, up to the first start at or past ip + 32.
+// An exclusive scan of the starts' lengths places each element in the output.
+// Each output byte of the round gets its source in a per-warp shared map: a
+// compressed position (literal) or an earlier output position (copy; an
+// overlapping copy repeats its first `offset` bytes).  A source inside the
+// round is followed through the map to a byte written before the round or a
+// literal byte, so that all bytes of a round are independent and the warp
+// writes them with one load and one store each.  A literal longer than 64
+// bytes (the last element of its round) is copied by the whole warp after
+// the round.  Every length and offset is checked against the piece's bounds;
+// a malformed block sets ERR_CORRUPT and stops.
+#define SNW_MAP 1024   // output bytes of one round: at most 16 elements of at most 64 bytes
+#define SNW_LONG 64    // literals longer than this are copied by the warp
+#define SNW_LIT 0x80000000u
+
+__device__ __forceinline__ void sn_warp_piece(const uint8_t *__restrict__ file, const InflateJob J, uint8_t *img, u32 *lvl,
+                                              Ctl *ctl, u32 *map, const int lane) {
+    const uint8_t *src = file + J.src;
+    uint8_t *dst = img + J.dst;
+    bool bad = false;
+    if (J.mode == 0) {
+        for (u32 i = lane; i < J.src_len; i += 32) dst[i] = src[i];
+    } else {
+        const u32 slen = J.src_len, dlen = J.dst_len;
+        u32 ip = 0, op = 0;
+        if (lane == 0) {  // the preamble: the uncompressed length
+            u64 ulen = 0;
+            int sh = 0;
+            for (;;) {
+                if (ip >= slen || sh > 28) {
+                    bad = true;
+                    break;
+                }
+                const uint8_t b = src[ip++];
+                ulen |= (u64)(b & 0x7f) << sh;
+                if (!(b & 0x80)) break;
+                sh += 7;
+            }
+            if (ulen != dlen) bad = true;
+        }
+        bad = __shfl_sync(FULL, (int)bad, 0) != 0;
+        ip = __shfl_sync(FULL, ip, 0);
+        while (!bad && op < dlen) {
+            if (ip >= slen) {
+                bad = true;
+                break;
+            }
+            // bytes [ip + lane, ip + lane + 8): lanes 0..10 load the aligned words over
+            // [ip, ip + 40) and the warp redistributes them
+            const uint8_t *blk = (const uint8_t *)((uintptr_t)(src + ip) & ~(uintptr_t)3);
+            u32 word = 0;
+            if (lane < 11) {
+                const uint8_t *wp = blk + 4 * lane;
+                if (blk >= src && blk + 44 <= src + slen) {
+                    word = __ldg((const u32 *)wp);
+                } else {
+                    for (int k = 0; k < 4; k++)
+                        if (wp + k >= src && wp + k < src + slen) word |= (u32)__ldg(wp + k) << (8 * k);
+                }
+            }
+            const u32 sh0 = (u32)((uintptr_t)(src + ip) & 3) + (u32)lane;
+            const u32 w0 = __shfl_sync(FULL, word, sh0 >> 2);
+            const u32 w1 = __shfl_sync(FULL, word, (sh0 >> 2) + 1);
+            const u32 w2 = __shfl_sync(FULL, word, (sh0 >> 2) + 2);
+            const u32 lo = __funnelshift_r(w0, w1, 8 * (sh0 & 3)), hi = __funnelshift_r(w1, w2, 8 * (sh0 & 3));
+            // the element a tag at ip + lane would be (selects, no branches)
+            const u32 tag = lo & 0xffu, t = tag & 3u, l6 = tag >> 2;
+            const u32 rest = (lo >> 8) | (hi << 24);  // bytes 1..4 after the tag
+            const u32 nb = l6 >= 60 ? l6 - 59 : 0;     // a literal's length bytes
+            const u32 lraw = nb ? rest & (0xffffffffu >> (32 - 8 * nb)) : l6;
+            const u32 hdr = t == 0 ? 1 + nb : (t == 1 ? 2 : (t == 2 ? 3 : 5));
+            const u32 len = t == 0 ? lraw + 1 : (t == 1 ? 4 + (l6 & 7u) : l6 + 1);  // 0 after a wrap
+            const u32 off = t == 1 ? ((tag >> 5) << 8) | (rest & 0xffu) : (t == 2 ? rest & 0xffffu : rest);
+            const u32 cs = t != 0 ? hdr : (lraw >= 0x7fff0000u ? 0x7fffffffu : hdr + lraw + 1);
+            // the chain of starts from ip
+            const u32 avail = min(32u, slen - ip);
+            u32 pos = 0, mask = 0;
+            while (pos < avail) {
+                mask |= 1u << pos;
+                pos += __shfl_sync(FULL, cs, pos);
+            }
+            const bool start = (mask >> lane) & 1u;
+            // lengths clamped in the scan (16 starts of at most 2^26 cannot wrap); the one
+            // element that may be longer, a long literal, is the round's last start
+            u32 mylen = start ? min(len, 1u << 26) : 0, incl = mylen;
+            for (int d = 1; d < 32; d <<= 1) {
+                const u32 y = __shfl_up_sync(FULL, incl, d);
+                if (lane >= d) incl += y;
+            }
+            const u32 excl = incl - mylen;  // round-relative output position
+            u32 total = __shfl_sync(FULL, incl, 31);
+            const u32 p = ip + (u32)lane;  // compressed position of this lane's tag
+            const u64 o = (u64)op + excl;
+            const bool live = start && o < dlen;  // elements after the last output byte are ignored
+            const bool mybad = live && ((u64)p + cs > slen || len == 0 || o + len > dlen ||
+                                        (t != 0 && (off == 0 || off > o)));
+            if (__any_sync(FULL, mybad)) {
+                bad = true;
+                break;
+            }
+            // outputs past dlen (trailing elements) and the long literal are not mapped
+            if (total > dlen - op) total = dlen - op;
+            const u32 lmask = __ballot_sync(FULL, live && t == 0 && len > SNW_LONG);
+            u32 mapped = total, lit_at = 0, lit_len = 0, lit_src = 0;
+            if (lmask) {
+                const int ll = __ffs(lmask) - 1;
+                mapped = __shfl_sync(FULL, excl, ll);
+                lit_len = __shfl_sync(FULL, len, ll);
+                lit_src = __shfl_sync(FULL, p + hdr, ll);
+                lit_at = op + mapped;
+                total = mapped + lit_len;
+            }
+            if (mapped > SNW_MAP) {  // unreachable: 16 starts of at most 64 bytes
+                bad = true;
+                break;
+            }
+            if (start && excl < mapped) {
+                // a literal's byte b comes from q + b; a copy's from o - off + (b mod off)
+                const u32 base = t == 0 ? SNW_LIT | (p + hdr) : (u32)o - off;
+                const u32 per = t == 0 ? 0xffffffffu : off;
+                for (u32 b = 0, r = 0; b < len; b++) {
+                    map[excl + b] = base + r;
+                    r = r + 1 == per ? 0 : r + 1;
+                }
+            }
+            __syncwarp();
+            for (u32 k = lane; k < mapped; k += 32) {
+                u32 s = map[k];
+                while (!(s & SNW_LIT) && s >= op) s = map[s - op];
+                dst[op + k] = (s & SNW_LIT) ? __ldg(src + (s & ~SNW_LIT)) : dst[s];
+            }
+            if (lit_len) {
+                for (u32 b = lane; b < lit_len; b += 32) dst[lit_at + b] = __ldg(src + lit_src + b);
+            }
+            __syncwarp();
+            op += total;
+            ip += pos;
+        }
+    }
+    if (bad && lane == 0) atomicOr(&ctl->err, (u32)ERR_CORRUPT);
+    __syncwarp();
+    if (lane == 0) x_level(J, dst, bad, lvl);
+}
+
+// Each warp claims pieces from a counter (zero at launch) until none is left.
+__global__ void __launch_bounds__(256) k_pq_inflate_small(const uint8_t *__restrict__ file, const InflateJob *jobs,
+                                                          uint32_t n, uint32_t *next, uint8_t *img, uint32_t *lvl,
+                                                          Ctl *ctl) {
+    __shared__ u32 s_map[8][SNW_MAP];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (;;) {
+        u32 j = 0;
+        if (lane == 0) j = atomicAdd(next, 1u);
+        j = __shfl_sync(FULL, j, 0);
+        if (j >= n) return;  // the whole warp
+        sn_warp_piece(file, jobs[j], img, lvl, ctl, s_map[warp], lane);
     }
 }
 
