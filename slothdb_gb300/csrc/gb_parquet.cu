@@ -523,6 +523,9 @@ struct RunJob {
 };
 
 #define PQ_WIN 16384
+#define RW_LONG_T 1024  // threads (an eighth of the bytes staged) of a walk of a long index stream
+#define RW_SHORT_T 128  // ... of one of up to RW_SHORT bytes, and of a level stream
+#define RW_SHORT 4096
 #define PQ_LEVEL_RUN 512  // bit-packed level runs are split at this many entries (bounds the popcount)
 
 // Run walk (RleDecoder::FetchRun, parquet.cpp:476-540), one CTA per stream.
@@ -541,19 +544,19 @@ struct RunJob {
 // popcount.  For a level stream, the page's defined entries must fit its
 // values (PLAIN: width bytes each); anything else sets ERR_CORRUPT.  Thread 0
 // walks it (bit width 1: few and long runs).
-constexpr int RW_T = 1024;
-constexpr int RW_B = 8192;          // bytes staged
-constexpr int RW_PER = RW_B / RW_T;
 constexpr int RW_HDR = 16;          // a header and an RLE value need no more
 constexpr uint32_t RW_FAR = 0xffff; // a jump that leaves what 16 bits hold
+constexpr int RW_PER = 8;           // bytes of a thread
 
+template <int T>
 struct RunWalk {
-    uint8_t win[RW_B + 32];
-    uint16_t jump[RW_B], even[RW_B], odd[RW_B];  // 1 run on; 2, then 8; 4
-    uint16_t entry[RW_B / 8 + 1];
-    uint32_t bits[RW_B / 32];
-    uint64_t warp_vals[RW_T / 32];
-    uint32_t warp_runs[RW_T / 32];
+    static constexpr int B = RW_PER * T;  // bytes staged
+    uint8_t win[B + 32];
+    uint16_t jump[B], even[B], odd[B];  // 1 run on; 2, then 8; 4
+    uint16_t entry[B / 8 + 1];
+    uint32_t bits[B / 32];
+    uint64_t warp_vals[T / 32];
+    uint32_t warp_runs[T / 32];
     uint32_t n_entry, bad, top;
     uint64_t next;
 };
@@ -579,8 +582,10 @@ __device__ __forceinline__ RunHead rw_head(const uint8_t *win, uint32_t i, uint3
     }
 }
 
+template <int T>
 __device__ __forceinline__ void rw_indices(const uint8_t *file, const RunJob &J, DRun *runs, uint32_t *page_runs,
-                                           Ctl *ctl, RunWalk &S) {
+                                           Ctl *ctl, RunWalk<T> &S) {
+    constexpr int RW_T = T, RW_B = RunWalk<T>::B;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t bw = J.bytes ? file[J.off] : 0, vb = (bw + 7) / 8;
     uint64_t pos = 1, vals = 0;
@@ -728,15 +733,23 @@ __device__ __forceinline__ void rw_indices(const uint8_t *file, const RunJob &J,
     }
 }
 
-__global__ void __launch_bounds__(RW_T) k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob *jobs, DRun *runs,
-                                                  uint32_t *page_runs, Ctl *ctl) {
+// Index streams of more than RW_SHORT bytes.
+__global__ void __launch_bounds__(RW_LONG_T) k_pq_runs_long(const uint8_t *file, const RunJob *jobs, DRun *runs,
+                                                            uint32_t *page_runs, Ctl *ctl) {
+    extern __shared__ __align__(16) unsigned char rw_smem[];
+    rw_indices<RW_LONG_T>(file, jobs[blockIdx.x], runs, page_runs, ctl, *(RunWalk<RW_LONG_T> *)rw_smem);
+}
+
+// Level streams and short index streams.
+__global__ void __launch_bounds__(RW_SHORT_T) k_pq_runs(const uint8_t *file, const DPage *pages, const RunJob *jobs,
+                                                        DRun *runs, uint32_t *page_runs, Ctl *ctl) {
     extern __shared__ __align__(16) unsigned char rw_smem[];
     uint8_t *win = rw_smem;      // levels: a window of the payload
     __shared__ uint64_t s_pos;   // stream position of the walk
     __shared__ uint32_t s_vals, s_runs, s_done, s_nn;
     const RunJob J = jobs[blockIdx.x];
     if (!J.levels) {
-        rw_indices(file, J, runs, page_runs, ctl, *(RunWalk *)rw_smem);
+        rw_indices<RW_SHORT_T>(file, J, runs, page_runs, ctl, *(RunWalk<RW_SHORT_T> *)rw_smem);
         return;
     }
     if (threadIdx.x == 0) {
@@ -871,18 +884,37 @@ __global__ void __launch_bounds__(RW_T) k_pq_runs(const uint8_t *file, const DPa
     }
 }
 
-// Run tables of the n streams at `jobs`.
-static cudaError_t launch_runs(size_t n, const uint8_t *file, const void *pages, const void *jobs, void *runs,
-                             void *page_runs, Ctl *ctl, cudaStream_t st) {
-    static_assert(sizeof(RunWalk) >= PQ_WIN, "a level window in the walk's memory");
-    static bool attr = false;
-    if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(k_pq_runs, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(RunWalk));
-        if (e) return e;
-        attr = true;
+static bool rw_is_long(const RunJob &j) { return !j.levels && j.bytes > RW_SHORT; }
+
+// Run tables of the streams `jobs`, whose device copy is dev_jobs: the long
+// ones lie behind the others (pq_page_table).
+static cudaError_t launch_runs(const std::vector<RunJob> &jobs, const uint8_t *file, const void *pages,
+                               const void *dev_jobs, void *runs, void *page_runs, Ctl *ctl, cudaStream_t st,
+                               int *launched = nullptr) {
+    static_assert(sizeof(RunWalk<RW_SHORT_T>) <= PQ_WIN + 16, "a short stream's walk in a level window");
+    size_t n = (size_t)(std::partition_point(jobs.begin(), jobs.end(), [](const RunJob &j) { return !rw_is_long(j); }) -
+                        jobs.begin());
+    // a few short streams beside long ones join them: no launch of their own
+    if (n < jobs.size() && n <= (size_t)sm_count() &&
+        std::none_of(jobs.begin(), jobs.begin() + n, [](const RunJob &j) { return j.levels != 0; }))
+        n = 0;
+    const size_t n_long = jobs.size() - n;
+    const RunJob *dj = (const RunJob *)dev_jobs;
+    if (launched) *launched = (n != 0) + (n_long != 0);
+    if (n_long) {
+        static bool attr = false;
+        if (!attr) {
+            const cudaError_t e = cudaFuncSetAttribute(k_pq_runs_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       sizeof(RunWalk<RW_LONG_T>));
+            if (e) return e;
+            attr = true;
+        }
+        k_pq_runs_long<<<(unsigned)n_long, RW_LONG_T, sizeof(RunWalk<RW_LONG_T>), st>>>(file, dj + n, (DRun *)runs,
+                                                                                     (uint32_t *)page_runs, ctl);
     }
-    k_pq_runs<<<(unsigned)n, RW_T, sizeof(RunWalk), st>>>(file, (const DPage *)pages, (const RunJob *)jobs, (DRun *)runs,
-                                                          (uint32_t *)page_runs, ctl);
+    if (n)
+        k_pq_runs<<<(unsigned)n, RW_SHORT_T, PQ_WIN + 16, st>>>(file, (const DPage *)pages, dj, (DRun *)runs,
+                                                                (uint32_t *)page_runs, ctl);
     return cudaGetLastError();
 }
 
@@ -1624,6 +1656,7 @@ static gb_status pq_page_table(const gb_pq_file *f, const PqView &V, uint32_t rg
             col_pages.push_back((uint32_t)pages.size());
         }
     }
+    std::stable_partition(jobs.begin(), jobs.end(), [](const RunJob &j) { return !rw_is_long(j); });
     return GB_OK;
 }
 
@@ -1662,7 +1695,7 @@ static gb_status pq_build_index(gb_pq_file *f, cudaStream_t st) {
         (e = cudaMemsetAsync(ctl, 0, sizeof(Ctl), st)))
         return fail(e, "cudaMemcpy (Parquet page index)");
     if (!jobs.empty()) {
-        if ((e = launch_runs(jobs.size(), (const uint8_t *)f->dev, f->idx_pages, dp, f->idx_runs, f->idx_page_runs,
+        if ((e = launch_runs(jobs, (const uint8_t *)f->dev, f->idx_pages, dp, f->idx_runs, f->idx_page_runs,
                              (Ctl *)ctl, st)))
             return fail(e, "k_pq_runs");
     }
@@ -1985,7 +2018,7 @@ gb_status gb_pq_dict_sum(gb_pq_file *f, uint32_t col, uint32_t rg_begin, uint32_
         return done(cuda_fail(e, "cudaMemcpyAsync (dictionary histogram)"));
     if (!jobs.empty()) {  // a batch's own run tables (the file in host memory)
         Ctl c;
-        if ((e = launch_runs(jobs.size(), dfile, d_pages, d_jobs, d_runs, d_page_runs, (Ctl *)d_ctl, st)) ||
+        if ((e = launch_runs(jobs, dfile, d_pages, d_jobs, d_runs, d_page_runs, (Ctl *)d_ctl, st)) ||
             (e = cudaMemcpyAsync(&c, d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st)) ||
             (e = cudaStreamSynchronize(st)))
             return done(cuda_fail(e, "k_pq_runs"));
@@ -2712,9 +2745,10 @@ extern "C" gb_status gb_agg_ingest_parquet(gb_agg *h, gb_pq_file *f, uint32_t rg
             GB_CUDA(cudaMemcpyAsync(S->dict_pages, jobs.data(), jobs.size() * sizeof(RunJob), cudaMemcpyHostToDevice,
                                     st));
             gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pq_runs", st);
-            GB_CUDA(launch_runs(jobs.size(), dfile, S->pages, S->dict_pages, S->runs, S->page_runs, dctl, st));
+            int launched = 0;
+            GB_CUDA(launch_runs(jobs, dfile, S->pages, S->dict_pages, S->runs, S->page_runs, dctl, st, &launched));
             gb_agg_prof_end(h, pm, st);
-            gb_agg_count_launch(h, 1);
+            gb_agg_count_launch(h, launched);
         }
         d_pages = S->pages;
         d_runs = S->runs;
