@@ -261,3 +261,15 @@ def test_small_pages_cost_no_more_than_large_ones():
     v = np.random.default_rng(1).integers(0, 10**6, n)
     small, large = (kernel_ms(plain(n, v, page_rows=r, codec="snappy"), "k_pq_inflate") for r in (200, 8192))
     assert small <= 2 * large, (small, large)
+
+
+def test_odd_pages_use_the_whole_gpu(monkeypatch):
+    """4,800 pages of three frames against 600 of them: with four decoding
+    warps an SM they took 8 rounds to one, with twenty 2."""
+    monkeypatch.setattr(pq, "zstd_compress", odd_frames(pq.zstd_compress, 1, "frames"))
+    rng = np.random.default_rng(2)
+    ms = []
+    for pages in (600, 4800):
+        v = rng.integers(0, 10**6, 500 * pages // 2)
+        ms.append(kernel_ms(plain(len(v), v, page_rows=500, codec="zstd"), "k_pz_"))
+    assert ms[1] <= 4 * ms[0], ms
