@@ -225,7 +225,11 @@ uint64_t gb_agg_row_groups_pruned(const gb_agg *h);
  *   "radix_bits"  log2 of the partition count, 6..12 (radix)
  *   "radix_precombine"  1 = the partition pass combines a warp's equal keys
  *                 before folding, 0 = folds tuple by tuple (radix; default 0
- *                 when every op is a DOUBLE SUM, else 1) */
+ *                 when every op is a DOUBLE SUM, else 1)
+ *   "zstd_scratch"  most bytes of scratch that the decode of a batch's ZSTD
+ *                 pages takes (0, the default: five for each page byte, at
+ *                 most 1.9 GB or what can be allocated); with less it decodes
+ *                 in smaller groups, at last with one lane per page */
 gb_status gb_agg_set_option(gb_agg *h, const char *name, int64_t value);
 /* 1 = radix mode, 0 = hash mode. */
 int32_t gb_agg_get_mode(const gb_agg *h);

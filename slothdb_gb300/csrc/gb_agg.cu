@@ -823,6 +823,7 @@ struct gb_agg {
     bool fast_ingest = true;      // integer plans take the register-resident fast kernel
     bool topn_small = true;       // K <= 32: warp-register TopN lists
     u32 tile_rows = 8192;
+    u64 zstd_scratch = 0;         // most bytes of the ZSTD page decode's scratch (0: what can be allocated)
     // profiling (CUDA events around each kernel, resolved at sync points)
     bool profiling = false;
     struct ProfEv { int stat; cudaEvent_t a, b; };
@@ -2584,6 +2585,9 @@ gb_status gb_agg_set_option(gb_agg *h, const char *name, int64_t value) {
     } else if (n == "fast_ingest") {
         if (value < 0 || value > 1) return GB_ERR_INVALID;
         h->fast_ingest = value != 0;
+    } else if (n == "zstd_scratch") {
+        if (value < 0) return GB_ERR_INVALID;
+        h->zstd_scratch = (u64)value;
     } else if (n == "ctas_per_sm") {
         if (value < 1 || value > 4) return GB_ERR_INVALID;
         h->ctas_per_sm = (int)value;
@@ -2744,6 +2748,7 @@ gb_status gb_agg_view(gb_agg *h, AggView *v) {
 }
 
 void gb_agg_count_launch(gb_agg *h, int n) { h->launches += (u64)n; }
+uint64_t gb_agg_zstd_scratch(const gb_agg *h) { return h->zstd_scratch; }
 
 void gb_agg_count_pruned(gb_agg *h, uint64_t n) { h->rg_pruned += n; }
 

@@ -2334,36 +2334,59 @@ static gb_status pq_unzstd(gb_agg *h, PqScratch *S, const uint8_t *dfile, std::v
         uint64_t bytes, blocks, full;
     };
     std::vector<Group> groups;
-    uint64_t most = 0, most_blocks = 0;
-    size_t most_n = 0;
     // many small pieces: without descriptors they are left to the serial decoder
     const bool small_serial = std::count_if(jobs.begin(), jobs.end(),
                                             [](const InflateJob &j) { return j.dst_len < PZ_SMALL; }) >= PZ_SMALL_MANY;
-    for (size_t k = 0; k < jobs.size();) {
-        Group g{k, 0, 0, 0, 0, 0};
-        for (; k < jobs.size() && (g.n == 0 || g.bytes + jobs[k].dst_len <= PZ_GROUP); k++, g.n++) {
-            jobs[k].aux = g.bytes;
-            jobs[k].blk = (uint32_t)g.blocks;
-            jobs[k].blk_cap = small_serial && jobs[k].dst_len < PZ_SMALL ? 0 : jobs[k].dst_len / 8192 + 4;
-            g.bytes += ((uint64_t)jobs[k].dst_len + 15) & ~15ull;
-            g.blocks += jobs[k].blk_cap;
-            g.full += jobs[k].dst_len / gbz::ZS_BLOCK_MAX + 1;
-            g.regular += jobs[k].blk_cap != 0;
+    // descriptors | block list | per piece: block count, odd mark | literals | sequences
+    auto up = [](uint64_t n) { return (n + 255) & ~255ull; };
+    uint64_t a_blk, a_list, a_nblk, a_odd, a_lit, a_seq, seqs, all;
+    size_t most_n;
+    // groups of up to `limit` page bytes (a piece at least; 0: all pieces are left to the serial decoder)
+    auto plan = [&](uint64_t limit) {
+        uint64_t most = 0, most_blocks = 0;
+        most_n = 0;
+        groups.clear();
+        for (size_t k = 0; k < jobs.size();) {
+            Group g{k, 0, 0, 0, 0, 0};
+            for (; k < jobs.size() && (g.n == 0 || !limit || g.bytes + jobs[k].dst_len <= limit); k++, g.n++) {
+                jobs[k].aux = g.bytes;
+                jobs[k].blk = (uint32_t)g.blocks;
+                jobs[k].blk_cap = !limit || (small_serial && jobs[k].dst_len < PZ_SMALL) ? 0 : jobs[k].dst_len / 8192 + 4;
+                if (!jobs[k].blk_cap) continue;
+                g.bytes += ((uint64_t)jobs[k].dst_len + 15) & ~15ull;
+                g.blocks += jobs[k].blk_cap;
+                g.full += jobs[k].dst_len / gbz::ZS_BLOCK_MAX + 1;
+                g.regular++;
+            }
+            most = std::max(most, g.bytes);
+            most_blocks = std::max(most_blocks, g.blocks);
+            most_n = std::max(most_n, g.n);
+            groups.push_back(g);
         }
-        most = std::max(most, g.bytes);
-        most_blocks = std::max(most_blocks, g.blocks);
-        most_n = std::max(most_n, g.n);
-        groups.push_back(g);
+        a_blk = up(sizeof(ZWork));
+        a_list = a_blk + up(most_blocks * sizeof(ZBlk));
+        a_nblk = a_list + up(most_blocks * 4);
+        a_odd = a_nblk + up(most_n * 4);
+        a_lit = a_odd + up(most_n * 4);
+        seqs = most / 3 + 1;
+        a_seq = a_lit + up(most);
+        all = a_seq + 3 * up(seqs * 4);
+        return most;
+    };
+    // where the scratch cannot be had: smaller groups, down to a piece each,
+    // then the serial decoder alone, which needs none
+    gb_status s;
+    const uint64_t at_most = gb_agg_zstd_scratch(h);
+    for (uint64_t limit = PZ_GROUP;;) {
+        const uint64_t most = plan(limit);
+        s = limit && at_most && all > at_most ? GB_ERR_OOM : grow(S->zwork, S->zwork_cap, all);
+        if (s == GB_OK) break;
+        if (s != GB_ERR_OOM || !limit) return s;
+        limit = most > jobs[0].dst_len + 16ull ? std::min(limit, most) / 2 : 0;
     }
     // a warp for every piece that may be left to it, up to the 20 an SM that decode at once
     const unsigned serial_blocks = (unsigned)std::min<size_t>((most_n + 3) / 4, (size_t)sm_count() * 5);
-    // descriptors | block list | per piece: block count, odd mark | literals | sequences
-    auto up = [](uint64_t n) { return (n + 255) & ~255ull; };
-    const uint64_t a_blk = up(sizeof(ZWork)), a_list = a_blk + up(most_blocks * sizeof(ZBlk)), a_nblk = a_list + up(most_blocks * 4),
-                   a_odd = a_nblk + up(most_n * 4), a_lit = a_odd + up(most_n * 4), seqs = most / 3 + 1,
-                   a_seq = a_lit + up(most), all = a_seq + 3 * up(seqs * 4);
-    gb_status s;
-    if ((s = grow(S->zjobs, S->zjobs_cap, jobs.size() * sizeof(InflateJob) + 16)) || (s = grow(S->zwork, S->zwork_cap, all)) ||
+    if ((s = grow(S->zjobs, S->zjobs_cap, jobs.size() * sizeof(InflateJob) + 16)) ||
         (s = grow(S->zscratch, S->zscratch_cap, (size_t)serial_blocks * 4 * sizeof(gbz::ZsScratch))))
         return s;
     static bool attr = false;

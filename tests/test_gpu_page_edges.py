@@ -273,3 +273,22 @@ def test_odd_pages_use_the_whole_gpu(monkeypatch):
         v = rng.integers(0, 10**6, 500 * pages // 2)
         ms.append(kernel_ms(plain(len(v), v, page_rows=500, codec="zstd"), "k_pz_"))
     assert ms[1] <= 4 * ms[0], ms
+
+
+@pytest.mark.parametrize("scratch", [0, 40 << 20, 9 << 20, 1_300_000, 100_000, 1])
+def test_zstd_scratch_that_is_short(scratch):
+    """24 pages of up to 200 KB: in one group, in several, in one for each page,
+    and with no scratch at all by the serial decoder."""
+    n = 300_000
+    rng = np.random.default_rng(6)
+    v = np.where(rng.random(n) < 0.6, rng.integers(0, 5000, n), 2**39)
+    prof = []
+    check(plain(n, v, page_rows=25_000, codec="zstd"), keys(n), v, options={"zstd_scratch": scratch}, profile=prof)
+    for p in prof:
+        groups = p["k_pz_blocks"][0]
+        if scratch == 0:
+            assert groups == 1 and p["k_pz_entropy"][0] == 1
+        elif scratch < 10**6:
+            assert groups == 1 and "k_pz_entropy" not in p
+        else:
+            assert groups == p["k_pz_entropy"][0] and (groups > 1) == (scratch < 20 << 20)
