@@ -1136,6 +1136,15 @@ static bool fast_ingest_plan(gb_agg *h, FastIngest &X);
 static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableRef &T, IngestArgs A, int grid,
                                     cudaStream_t st);
 
+// A spill buffer of at least `records` records.
+static gb_status spill_ensure(gb_agg *h, u64 records) {
+    if (h->spill_cap >= records) return GB_OK;
+    h->spill_cap = 0;  // a failed allocation leaves none
+    gb_status s = h->spill.ensure((size_t)records * (1 + h->plan.words) * 8);
+    if (s == GB_OK) h->spill_cap = (u32)records;
+    return s;
+}
+
 static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
     if (n_rows == 0) return GB_OK;
     if (h->plan.n_dist) {
@@ -1162,20 +1171,25 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
         const u64 tr = (n_rows + max_ctas * each - 1) / (max_ctas * each);
         tile_rows = (u32)std::max<u64>(1024, (tr + 511) / 512 * 512);
     }
-    const u64 n_tiles_total = (n_rows + tile_rows - 1) / tile_rows;
-    int grid = (int)std::min<u64>((u64)max_ctas, n_tiles_total);
     // the shared table pays when the estimated groups fit it; past that every
     // row would probe a full table before its HBM fold
     int S = h->smem_slots;
     if (h->est_groups > (u64)S) S = 0;
     size_t smem = (size_t)S * 8 * (1 + words);
-    // spill capacity: threshold + what in-flight tiles and the final flush can add
-    u64 margin = (u64)grid * (2 * (u64)tile_rows + (u64)S) + 1024;
-    u64 need_cap = (1u << 20) + margin;
-    if (h->spill_cap < need_cap) {
-        gb_status s = h->spill.ensure((size_t)need_cap * (1 + words) * 8);
-        if (s) return s;
-        h->spill_cap = (u32)need_cap;
+    // spill capacity: threshold + what in-flight tiles (a CTA of the fast path
+    // has claimed its next one too) and the final flush can add, a row of its own
+    // for each record.  Where it cannot be had, with tiles of half the rows
+    u64 n_tiles_total, margin;
+    int grid;
+    for (;;) {
+        n_tiles_total = (n_rows + tile_rows - 1) / tile_rows;
+        grid = (int)std::min<u64>((u64)max_ctas, n_tiles_total);
+        margin = std::min<u64>((u64)grid * ((fast ? 2 : 1) * (u64)tile_rows + (u64)S), n_rows) + 1024;
+        const u64 need_cap = (1u << 20) + margin;
+        const gb_status s = spill_ensure(h, need_cap);
+        if (s == GB_OK) break;
+        if (s != GB_ERR_OOM || !fast || tile_rows < 2048) return s;
+        tile_rows /= 2;
     }
     h->spill_threshold = (u32)(h->spill_cap - margin);
     static bool attr_set[2] = {false, false};
@@ -1434,11 +1448,7 @@ static gb_status radix_emit(gb_agg *h, cudaStream_t st) {
     // a partition whose groups overflow its shared table folds the rest into
     // the HBM table, which spills (at most once per tuple) when full
     {
-        const u64 need = tuples + 4096;
-        if (h->spill_cap < need) {
-            if ((s = h->spill.ensure((size_t)need * (1 + h->plan.words) * 8))) return s;
-            h->spill_cap = (u32)need;
-        }
+        if ((s = spill_ensure(h, tuples + 4096))) return s;
         h->spill_threshold = h->spill_cap;
     }
     for (size_t c = 0; c < h->out_valid.size(); c++)

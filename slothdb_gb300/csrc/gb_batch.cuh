@@ -1095,12 +1095,7 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
             for (u64 c = 0; c * 8192 < n; c++) it_str.push_back({q, (u32)c});
         }
         // HBM table, spill buffer, outputs of the handle
-        const int words = h->plan.words;
-        const u64 need_spill = (1u << 16) + 4096;
-        if (h->spill_cap < need_spill) {
-            if ((s = h->spill.ensure((size_t)need_spill * (1 + words) * 8))) return s;
-            h->spill_cap = (u32)need_spill;
-        }
+        if ((s = spill_ensure(h, (1u << 16) + 4096))) return s;
         if ((s = alloc_outputs(h, h->cap + 2))) return s;
         if (h->plan.n_dist) {
             // pair sets for this query's rows, emptied by the batch's init
