@@ -1192,12 +1192,11 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
         tile_rows /= 2;
     }
     h->spill_threshold = (u32)(h->spill_cap - margin);
-    static bool attr_set[2] = {false, false};
-    if (!attr_set[0]) {
-        cudaFuncSetAttribute(k_ingest<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_ingest<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        attr_set[0] = attr_set[1] = true;
-    }
+    static OncePerDevice attr;
+    GB_CUDA(attr([] {
+        const cudaError_t e = allow_smem(k_ingest<true>, 200 * 1024);
+        return e ? e : allow_smem(k_ingest<false>, 200 * 1024);
+    }));
     u64 first = 0;
     while (first < n_tiles_total) {
         if (!h->ctl_clean) GB_CUDA(cudaMemsetAsync(&dctl->spill_count, 0, 4 * 4, st));  // spill_count, tile_counter, stop, err
@@ -1972,11 +1971,8 @@ static gb_status run_topn(gb_agg *h, cudaStream_t st) {
     int sortn = (int)next_pow2((u64)2 * K);
     if (sortn < 1024) sortn = 1024;
     size_t smem = (size_t)sortn * (8 + 8 + 4);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_topn, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-        attr = true;
-    }
+    static OncePerDevice attr;
+    GB_CUDA(attr([] { return allow_smem(k_topn, 100 * 1024); }));
     int grid = (int)std::min<u64>((u64)sm_count() * 2, std::max<u64>(1, n / 4096));
     gb_status s;
     if ((s = h->topn_ids_a.ensure((size_t)grid * K * 4))) return s;

@@ -1011,23 +1011,17 @@ static gb_status launch_ingest_fast(gb_agg *h, const FastIngest &X, const TableR
     A.match_least = h->precombine_set ? (h->precombine ? 0 : 33) : (S == 0 ? MATCH_HBM : (F.sums_f ? MATCH_SHARED : 33));
     A.smem_slots = S;
     const size_t smem = FAST_SMEM(S, F.swords);
-    static bool attr_set = false;
-    if (!attr_set) {
-        for (int a = 0; a < 2; a++)
-            for (int n = 0; n <= FAST_MAX_OPS; n++)
-                for (int u = 0; u < 2; u++)
-                    for (int f = 0; f < 2; f++)
-                        GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel(a, n, u, f),
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        for (int n = 1; n <= FAST_MAX_OPS; n++)
-            GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel_f(n), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         200 * 1024));
-        for (int f = 0; f < 2; f++)
-            for (int n = 1 + f; n <= FAST_MAX_OPS; n++)
-                GB_CUDA(cudaFuncSetAttribute(fast_ingest_kernel_d(f, n), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             200 * 1024));
-        attr_set = true;
-    }
+    static OncePerDevice attr;
+    GB_CUDA(attr([] {
+        const size_t most = 200 * 1024;
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < 8 * (FAST_MAX_OPS + 1) && !e; i++)
+            e = allow_smem(fast_ingest_kernel(i & 1, i >> 3, (i >> 1) & 1, (i >> 2) & 1), most);
+        for (int n = 1; n <= FAST_MAX_OPS && !e; n++)
+            if (!(e = allow_smem(fast_ingest_kernel_f(n), most)) && !(e = allow_smem(fast_ingest_kernel_d(0, n), most)) && n > 1)
+                e = allow_smem(fast_ingest_kernel_d(1, n), most);
+        return e;
+    }));
     {
         ProfScope ps(h, "k_ingest_fast", st);
         const FastIngestKernel k = F.dist ? fast_ingest_kernel_d(F.flt, F.n_ops)
@@ -1210,12 +1204,12 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
     b->n_str = (u32)it_str.size();
     b->n_ingest = (u32)it_ing.size();
     b->n_compact = (u32)it_cmp.size();
-    static bool attr = false;
-    if (!attr) {
-        for (int c = 0; c < BATCH_CLASSES; c++)
-            cudaFuncSetAttribute(batch_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024 + 256);
-        attr = true;
-    }
+    static OncePerDevice attr;
+    GB_CUDA(attr([] {
+        cudaError_t e = cudaSuccess;
+        for (int c = 0; c < BATCH_CLASSES && !e; c++) e = allow_smem(batch_kernel(c), 96 * 1024 + 256);
+        return e;
+    }));
     b->prepared = true;
     return GB_OK;
 }

@@ -263,7 +263,12 @@ __device__ __forceinline__ void op_apply(int kind, u64 *w, u64 v, u64 ident) {
 // ----------------------------------------------------------------- host side
 #ifndef __CUDACC_RTC__
 #include <string>
+#include "gb_once.h"
 namespace gb {
+template <class K>
+inline cudaError_t allow_smem(K kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 void set_error(const char *fmt, ...);
 gb_status cuda_fail(cudaError_t e, const char *what);
 int sm_count();

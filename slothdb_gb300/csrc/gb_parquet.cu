@@ -902,13 +902,8 @@ static cudaError_t launch_runs(const std::vector<RunJob> &jobs, const uint8_t *f
     const RunJob *dj = (const RunJob *)dev_jobs;
     if (launched) *launched = (n != 0) + (n_long != 0);
     if (n_long) {
-        static bool attr = false;
-        if (!attr) {
-            const cudaError_t e = cudaFuncSetAttribute(k_pq_runs_long, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       sizeof(RunWalk<RW_LONG_T>));
-            if (e) return e;
-            attr = true;
-        }
+        static OncePerDevice attr;
+        if (const cudaError_t e = attr([] { return allow_smem(k_pq_runs_long, sizeof(RunWalk<RW_LONG_T>)); })) return e;
         k_pq_runs_long<<<(unsigned)n_long, RW_LONG_T, sizeof(RunWalk<RW_LONG_T>), st>>>(file, dj + n, (DRun *)runs,
                                                                                      (uint32_t *)page_runs, ctl);
     }
@@ -2389,11 +2384,8 @@ static gb_status pq_unzstd(gb_agg *h, PqScratch *S, const uint8_t *dfile, std::v
     if ((s = grow(S->zjobs, S->zjobs_cap, jobs.size() * sizeof(InflateJob) + 16)) ||
         (s = grow(S->zscratch, S->zscratch_cap, (size_t)serial_blocks * 4 * sizeof(gbz::ZsScratch))))
         return s;
-    static bool attr = false;
-    if (!attr) {
-        GB_CUDA(cudaFuncSetAttribute(k_pz_bytes, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ZByteShared)));
-        attr = true;
-    }
+    static OncePerDevice attr;
+    GB_CUDA(attr([] { return allow_smem(k_pz_bytes, sizeof(ZByteShared)); }));
     GB_CUDA(cudaMemcpyAsync(S->zjobs, jobs.data(), jobs.size() * sizeof(InflateJob), cudaMemcpyHostToDevice, st));
     for (const Group &g : groups) {
         uint8_t *z = (uint8_t *)S->zwork;
@@ -2544,11 +2536,8 @@ static gb_status pq_inflate_batch(gb_agg *h, const gb_pq_file *f, PqScratch *S, 
     if (n_pieces)
         GB_CUDA(cudaMemcpyAsync(S->ijobs, jobs.data(), jobs.size() * sizeof(InflateJob), cudaMemcpyHostToDevice, st));
     if (n_jobs) {
-        static bool attr = false;
-        if (!attr) {
-            GB_CUDA(cudaFuncSetAttribute(k_pq_inflate, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SnapShared)));
-            attr = true;
-        }
+        static OncePerDevice attr;
+        GB_CUDA(attr([] { return allow_smem(k_pq_inflate, sizeof(SnapShared)); }));
         gb_prof_mark *pm = gb_agg_prof_begin(h, "k_pq_inflate", st);
         const unsigned grid = (unsigned)std::min<size_t>(n_jobs, (size_t)sm_count() * X_CTAS);
         k_pq_inflate<<<grid, XT, sizeof(SnapShared), st>>>(dfile, (const InflateJob *)S->ijobs, (uint32_t)n_jobs, next,

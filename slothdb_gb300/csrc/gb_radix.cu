@@ -1400,9 +1400,7 @@ static P2Fn g_p2[4 * (RADIX_MAX_OPS + 1)];
 static P1Fn g_p1_spec[2][2];  // specialised P1: BIGINT key, one SUM [integer, DOUBLE][predicate]
 static P2Fn g_p2_gw[RADIX_MAX_OPS + 1];  // P2 with the state words in L2 (ops all DOUBLE SUM), one value column
 
-static gb_status radix_set_attributes() {
-    static bool done = false;
-    if (done) return GB_OK;
+static gb_status radix_set_attributes_here() {
     fill_tables<1>(g_p1, g_p2);
     fill_tables<2>(g_p1, g_p2);
     fill_tables<3>(g_p1, g_p2);
@@ -1423,8 +1421,14 @@ static gb_status radix_set_attributes() {
             if ((s = allow_max_smem(g_p1[v * (RADIX_MAX_OPS + 1) + o]))) return s;
             if ((s = allow_max_smem(g_p2[v * (RADIX_MAX_OPS + 1) + o]))) return s;
         }
-    done = true;
     return GB_OK;
+}
+
+static gb_status radix_set_attributes() {
+    static OncePerDevice once;
+    gb_status s = GB_OK;
+    const cudaError_t e = once([&] { return (s = radix_set_attributes_here()) ? cudaErrorUnknown : cudaSuccess; });
+    return s || !e ? s : cuda_fail(e, "cudaGetDevice");
 }
 
 gb_status radix_launch_p1(const Plan &P, const RadixPlan &R, const RadixRef &X, const TableRef &T,
