@@ -157,9 +157,10 @@ int gb_abi_version(void);
 gb_status gb_agg_create(const gb_agg_spec *spec, gb_agg **out);
 
 /* Device bytes a GROUP BY of `nrows` rows with this spec is expected to hold
- * (hash table sized from min(est_groups, nrows), result columns, spill
- * records, string dictionary).  Compiles the plan only; allocates nothing.
- * Used for admission control; no reference counterpart. */
+ * in a batch (hash table sized from min(est_groups, nrows), result columns,
+ * spill records, string dictionary; a handle of its own keeps tables of up to
+ * 65,536 groups sparser).  Compiles the plan only; allocates nothing.  Used for
+ * admission control; no reference counterpart. */
 gb_status gb_agg_estimate_bytes(const gb_agg_spec *spec, uint64_t nrows, uint64_t *bytes);
 
 /* Replaces the handle's WHERE predicates (same plan otherwise), after create

@@ -686,6 +686,19 @@ static u64 table_cap(u64 est) {
     return std::max<u64>(1024, next_pow2(est * f));
 }
 
+// Two slots a group at least.
+static u64 table_cap_dense(u64 est) { return std::max<u64>(1024, next_pow2(est * 2)); }
+
+// ... and of a query of n rows in a batch, whose tables are emptied and read one
+// with the other: sparse only where each slot serves 8 rows or more (init +
+// ingest + compact: 64 queries of 50,000 rows and 8,000 groups sparse 311 us, dense
+// 193; 16 of 50,000 and 1,000 groups 80 and 93; one of 10M and 30,000 350 and 366).
+static u64 table_cap_batch(u64 est, u64 n) {
+    u64 cap = table_cap(est);
+    while (cap > table_cap_dense(est) && cap > n / 8) cap >>= 1;
+    return cap;
+}
+
 // Words of a table: cap + 2 states, then cap keys.
 static u64 table_words(const Plan &P, u64 cap) { return (cap + 2) * (u64)P.stride + cap; }
 
@@ -2023,6 +2036,8 @@ static gb_status run_topn(gb_agg *h, cudaStream_t st) {
     return GB_OK;
 }
 
+static gb_status agg_create(const gb_agg_spec *spec, u64 batch_rows, gb_agg **out);
+
 // =================================================================== C ABI
 extern "C" {
 
@@ -2045,11 +2060,11 @@ gb_status gb_agg_estimate_bytes(const gb_agg_spec *spec, uint64_t nrows, uint64_
     if (s) return s;
     const u64 est = std::max<u64>(1, std::min<u64>(spec->est_groups ? spec->est_groups : (1u << 15),
                                                    std::max<u64>(nrows, 1)));
-    const u64 cap = table_cap(est);
+    const u64 cap = table_cap_dense(est);
     u64 b = table_words(h.plan, cap) * 8;                               // hash table
     for (int t : h.out_types) b += (cap + 2) * (u64)(t == GB_T_VARCHAR ? 8 : type_size(t)) + (cap + 2) / 8;
     b += (u64)((1u << 16) + 4096) * (1 + h.plan.words) * 8;            // spill records
-    if (h.str_col >= 0) b += 4 * 2 * cap * 8 + 40 * est + 16 * est;    // dictionary, arena, emitted strings
+    if (h.str_col >= 0) b += 4 * table_cap(est) * 8 + 40 * est + 16 * est;  // dictionary, arena, emitted strings
     if (h.plan.n_dist)                                                   // (group, value) pair sets
         b += std::max<u64>(1024, next_pow2(2 * std::max<u64>(nrows, 1))) * 16 * h.plan.n_dist *
              (h.dist_null_sets ? 2 : 1);
@@ -2085,7 +2100,12 @@ gb_status gb_agg_set_filters(gb_agg *h, const gb_filter *filters, uint32_t n_fil
     return GB_OK;
 }
 
-gb_status gb_agg_create(const gb_agg_spec *spec, gb_agg **out) {
+gb_status gb_agg_create(const gb_agg_spec *spec, gb_agg **out) { return agg_create(spec, 0, out); }
+
+}  // extern "C"
+
+// batch_rows: of a query in a batch (0: a handle of its own).
+static gb_status agg_create(const gb_agg_spec *spec, u64 batch_rows, gb_agg **out) {
     if (!spec || !out) {
         set_error("null spec/out");
         return GB_ERR_INVALID;
@@ -2110,7 +2130,7 @@ gb_status gb_agg_create(const gb_agg_spec *spec, gb_agg **out) {
     }
     gb_apply_tuning(h);
     u64 est = h->est_groups ? h->est_groups : (1u << 15);
-    h->cap = h->mode == 1 ? 4096 : table_cap(est);
+    h->cap = h->mode == 1 ? 4096 : batch_rows ? table_cap_batch(est, batch_rows) : table_cap(est);
     if ((s = h->ctl_buf.ensure(sizeof(Ctl)))) {
         delete h;
         return s;
@@ -2134,6 +2154,8 @@ gb_status gb_agg_create(const gb_agg_spec *spec, gb_agg **out) {
     *out = h;
     return GB_OK;
 }
+
+extern "C" {
 
 gb_status gb_agg_set_topn(gb_agg *h, uint32_t col_idx, int32_t ascending, uint64_t limit) {
     if (!h) return GB_ERR_INVALID;

@@ -1125,8 +1125,15 @@ static gb_status batch_prepare(gb_batch *b, cudaStream_t st) {
             d.init_words += sw * (h->plan.null_sets ? 2 : 1) + 2 + GB_MAX_DISTINCT;
         }
         for (u64 c = 0; c * INIT_WORDS < d.init_words; c++) it_init.push_back({q, (u32)c});
+        // rows straight to the HBM table: tiles so small that the CTAs work on one
+        // query's table at a time (3 queries of 2M rows and 1.5M groups, ingest: tiles
+        // of 16,384 rows 603 us, one for each CTA 401)
         d.tile_rows = b->tile_rows;
-        for (u64 c = 0; c * b->tile_rows < n; c++) it_ing.push_back({q, (u32)c});
+        if (d.smem_slots == 0) {
+            const u64 ctas = (u64)sm_count() * b->ctas_per_sm;
+            d.tile_rows = (u32)std::min<u64>(b->tile_rows, std::max<u64>(2048, ((n + ctas - 1) / ctas + 511) / 512 * 512));
+        }
+        for (u64 c = 0; c * d.tile_rows < n; c++) it_ing.push_back({q, (u32)c});
         for (u64 c = 0; c * (COMPACT_PER * 256) < h->cap + 2; c++) it_cmp.push_back({q, (u32)c});
         if (d.is_str) {
             // string results for up to out_cap groups; their bytes are at most
@@ -1378,7 +1385,7 @@ gb_status gb_batch_add(gb_batch *b, const gb_agg_spec *spec, const gb_col *cols,
     sp.est_groups = std::max<u64>(1, std::min<u64>(est, nrows));
     gb_agg *h = nullptr;
     gb_status s;
-    const std::string key = batch_pool_key(sp, table_cap(sp.est_groups));
+    const std::string key = batch_pool_key(sp, table_cap_batch(sp.est_groups, nrows));
     auto it = b->pool.find(key);
     if (it != b->pool.end()) {
         // an idle handle of the same plan shape and table size: rebind it
@@ -1403,10 +1410,10 @@ gb_status gb_batch_add(gb_batch *b, const gb_agg_spec *spec, const gb_col *cols,
         if (qidx) *qidx = (uint32_t)(b->handles.size() - 1);
         return GB_OK;
     }
-    if ((s = gb_agg_create(&sp, &h))) return s;
+    if ((s = agg_create(&sp, std::max<u64>(nrows, 1), &h))) return s;
     if (h->mode == 1) {  // the batch runs the hash pipeline for every query
         h->mode = 0;
-        h->cap = table_cap(h->est_groups ? h->est_groups : (1u << 15));
+        h->cap = table_cap_batch(h->est_groups, nrows);
         if ((s = init_table(h, h->table, h->cap, 0)) || (s = cuda_sync_legacy())) {
             gb_agg_destroy(h);
             return s;
