@@ -893,9 +893,9 @@ static FastPlan make_fast_plan(const Plan &P, FastFilters &FF, int max_ops = BAT
 }
 
 // ----------------------------------------------------- single-query fast ingest
-// The hash ingest of one query whose plan compiles into registers (integer
-// keys and ops, up to FAST_MAX_OPS ops and FAST_MAX_FILTERS numeric
-// predicates): the batch's fast tile path as a persistent kernel over the
+// The hash ingest of one query whose plan compiles into registers (integer or
+// string-id keys, integer, DOUBLE and COUNT(DISTINCT) ops, up to FAST_MAX_OPS of
+// them and FAST_MAX_FILTERS numeric predicates): the batch's fast tile path as a persistent kernel over the
 // query's tiles, with one narrow shared table per CTA for the whole launch
 // and spill records instead of re-runs.  Same tile-claim / spill-threshold
 // protocol as k_ingest, so run_ingest drives both.
@@ -956,7 +956,8 @@ typedef void (*FastIngestKernel)(Plan, FastPlan, FastFilters, TableRef, IngestAr
     }
 
 // Plans with DOUBLE ops: one kernel for each number of ops, with the NULL,
-// predicate and key match code whether they need it or not.
+// predicate and key match code whether they need it or not (4M rows without
+// either, 1,000 groups: SUM 57 us, 49 without that code; three ops 94 and 90).
 static FastIngestKernel fast_ingest_kernel_f(int nops) {
     static const FastIngestKernel tab[FAST_MAX_OPS] = {
         k_ingest_fast<MATCH_ASK, 1, true, true, true>, k_ingest_fast<MATCH_ASK, 2, true, true, true>,

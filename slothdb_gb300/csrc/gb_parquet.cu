@@ -7,8 +7,9 @@
 // ReadColumnInto's page loop).
 //
 // Device, per batch of row groups:
-//   k_pq_runs   one CTA per dictionary-encoded data page: the page is staged in
-//               shared memory and its RLE / bit-packed run headers are walked
+//   k_pq_runs   one CTA per dictionary-encoded data page (and per level stream),
+//               128 or 1,024 threads by the stream's length: the page is staged
+//               in shared memory and its RLE / bit-packed run headers are walked
 //               into a run table (RleDecoder::FetchRun, parquet.cpp:485-512).
 //   k_pq_views  per row chunk: each column's pages over the chunk and the run
 //               window of the dictionary column the scan stages (searched for
@@ -531,12 +532,15 @@ struct RunJob {
 // Run walk (RleDecoder::FetchRun, parquet.cpp:476-540), one CTA per stream.
 //
 // Dictionary indices: where a run starts is known only from the one before
-// it, so the walk is one chain of headers.  The CTA stages RW_B bytes, takes
+// it, so the walk is one chain of headers.  The CTA stages eight bytes a thread, takes
 // every byte as a header and notes where its run would end, doubles these
 // jumps three times (8 runs on), and one thread follows the long jumps; the
 // starts they pass expand in parallel, and a scan of the runs' entries places
-// them.  128 pages of 65,536 entries (130 KB, ~4,400 runs each): 570 us with
-// one thread walking header after header.
+// them.  128 pages of 65,536 entries (130 KB, ~4,400 runs each): 170 us; 570
+// with one thread walking header after header.  A block of 1,024 threads takes
+// ~10 us for the shortest stream, two on an SM: short ones have 128 threads
+// (10,000 streams of 250 bytes 378 -> 41 us, 2,000 of 1.3 KB 94 -> 20, 800 of
+// 3.1 KB 52 -> 25; 286 of 8.8 KB 37 with 1,024 threads, 70 with 128).
 //
 // A level stream's runs also carry the defined entries before them, and its
 // bit-packed runs are split every PQ_LEVEL_RUN entries so that a row's
