@@ -1206,10 +1206,11 @@ static gb_status run_ingest(gb_agg *h, u64 n_rows, cudaStream_t st) {
     }
     h->spill_threshold = (u32)(h->spill_cap - margin);
     static OncePerDevice attr;
-    GB_CUDA(attr([] {
-        const cudaError_t e = allow_smem(k_ingest<true>, 200 * 1024);
-        return e ? e : allow_smem(k_ingest<false>, 200 * 1024);
-    }));
+    if (!fast)
+        GB_CUDA(attr([] {
+            const cudaError_t e = allow_smem(k_ingest<true>, 200 * 1024);
+            return e ? e : allow_smem(k_ingest<false>, 200 * 1024);
+        }));
     u64 first = 0;
     while (first < n_tiles_total) {
         if (!h->ctl_clean) GB_CUDA(cudaMemsetAsync(&dctl->spill_count, 0, 4 * 4, st));  // spill_count, tile_counter, stop, err
